@@ -14,7 +14,9 @@ The reference's tables.h is looked for, in order, at: the first argument; $KF_MC
 (a path to tables.h); $KF_REFERENCE_DIR/include/tables.h (a checkout of the reference);
 baseline/_ref/include/tables.h under the repository root; include/tables.h of a checkout
 named `reference` beside the repository.  When none exists, a previously generated
-header is kept; with neither, the script stops with an error naming these places.
+header is kept; with neither, the tables are derived from the cube's geometry (derive()):
+the same corner and edge numbering, edge masks and triangle counts, with this project's own
+choice of diagonals inside each polygon.
 """
 from __future__ import annotations
 
@@ -94,6 +96,118 @@ def check(t: dict[str, list[int]]) -> None:
     assert sum(t["ntri"]) == 820
 
 
+# Corners in the classic path's numbering (marchingCubes.cs:142-150) and the corner pairs of
+# the 12 edges; a face is its four corners in cyclic order.
+CORNERS = [(0, 0, 0), (1, 0, 0), (1, 1, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1), (1, 1, 1), (0, 1, 1)]
+EDGES = [(0, 1), (1, 2), (2, 3), (3, 0), (4, 5), (5, 6), (6, 7), (7, 4), (0, 4), (1, 5), (2, 6), (3, 7)]
+FACES = [(0, 1, 2, 3), (4, 5, 6, 7), (0, 1, 5, 4), (3, 2, 6, 7), (0, 3, 7, 4), (1, 2, 6, 5)]
+
+
+def _edge(a: int, b: int) -> int:
+    return next(e for e, p in enumerate(EDGES) if set(p) == {a, b})
+
+
+def _segments(case: int) -> list[tuple[int, int]]:
+    """The contour on each face, as pairs of cut edges: every run of set corners along the
+    face's cycle is cut off by one segment (so two set corners on a diagonal stay separate,
+    in both cubes that share the face)."""
+    segs = []
+    for f in FACES:
+        inside = [(case >> c) & 1 for c in f]
+        if sum(inside) in (0, 4):
+            continue
+        for k in range(4):
+            if inside[k] and not inside[k - 1]:  # a run of set corners starts here
+                j = k
+                while inside[(j + 1) % 4]:
+                    j = (j + 1) % 4
+                segs.append((_edge(f[k - 1], f[k]), _edge(f[j], f[(j + 1) % 4])))
+    return segs
+
+
+def _loops(segs: list[tuple[int, int]]) -> list[list[int]]:
+    """The face segments joined into closed polygons, each from its lowest edge."""
+    left, loops = list(segs), []
+    while left:
+        a, b = left.pop(min(range(len(left)), key=lambda i: min(left[i])))
+        loop = [min(a, b), max(a, b)]
+        while loop[0] != loop[-1]:
+            i = next(i for i, s in enumerate(left) if loop[-1] in s)
+            s = left.pop(i)
+            loop.append(s[1] if s[0] == loop[-1] else s[0])
+        loops.append(loop[:-1])
+    return loops
+
+
+def _midpoint(e: int) -> list[float]:
+    p, q = (CORNERS[c] for c in EDGES[e])
+    return [0.5 * (p[k] + q[k]) for k in range(3)]
+
+
+def _winding(case: int, loop: list[int]) -> float:
+    """Sign of the loop's area vector along its own free-space direction (the sum over its
+    edges of clear corner - set corner)."""
+    m = [_midpoint(e) for e in loop]
+    area, out = [0.0] * 3, [0.0] * 3
+    for i, e in enumerate(loop):
+        u, v = m[i], m[(i + 1) % len(loop)]
+        a, b = EDGES[e]
+        s, c = (a, b) if (case >> a) & 1 else (b, a)
+        for k in range(3):
+            area[k] += u[(k + 1) % 3] * v[(k + 2) % 3] - u[(k + 2) % 3] * v[(k + 1) % 3]
+            out[k] += CORNERS[c][k] - CORNERS[s][k]
+    return sum(area[k] * out[k] for k in range(3))
+
+
+def _triangulate(loop: list[int]) -> list[tuple[int, int, int]] | None:
+    """Triangles of a polygon whose diagonals never join two edges of one cube face (such a
+    diagonal would lie in the face, where the neighbour cube's polygon has its own side)."""
+    def allowed(a, b):
+        ca, cb = EDGES[a], EDGES[b]
+        return not any(set(ca) <= set(f) and set(cb) <= set(f) for f in FACES)
+
+    if len(loop) == 3:
+        return [(loop[0], loop[1], loop[2])]
+    n = len(loop)
+    for k in range(1, n - 1):  # the triangle on the side (loop[0], loop[-1]) and its apex
+        if (k > 1 and not allowed(loop[0], loop[k])) or (k < n - 2 and not allowed(loop[k], loop[-1])):
+            continue
+        lo = _triangulate(loop[:k + 1]) if k > 1 else []
+        hi = _triangulate(loop[k:]) if k < n - 2 else []
+        if lo is not None and hi is not None:
+            return [(loop[0], loop[k], loop[-1])] + lo + hi
+    return None
+
+
+def derive() -> dict[str, list[int]]:
+    """The case tables from the cube's geometry: on every face the contour cuts off each run
+    of set corners, the face segments close into polygons, each polygon is triangulated and
+    wound clockwise seen from the clear (free-space) corners.  offsets3 holds the edges' end
+    points with y and z swapped (histoPyramids.cs:27-36)."""
+    t = {"edge": [], "tri": [], "nverts": [], "ntri": [], "offsets3": []}
+    for case in range(256):
+        mask = sum(1 << e for e, (a, b) in enumerate(EDGES) if ((case >> a) ^ (case >> b)) & 1)
+        row = []
+        for loop in _loops(_segments(case)):
+            if _winding(case, loop) > 0:
+                loop = [loop[0]] + loop[:0:-1]
+            tris = _triangulate(loop)
+            if tris is None:
+                raise ValueError(f"case {case}: no triangulation of {loop}")
+            for tri in tris:
+                row += tri
+        t["edge"].append(mask)
+        t["tri"] += row + [255] * (16 - len(row))
+        t["nverts"].append(len(row))
+        t["ntri"].append(len(row) // 3)
+    for a, b in EDGES:
+        for c in (a, b):
+            x, y, z = CORNERS[c]
+            t["offsets3"] += [x, z, y]
+    check(t)
+    return t
+
+
 def emit(t: dict[str, list[int]], out: str) -> None:
     os.makedirs(os.path.dirname(out), exist_ok=True)
 
@@ -126,11 +240,12 @@ def main(argv: list[str]) -> int:
         if os.path.exists(out):
             print(f"gen_mc_tables: no tables.h found; keeping existing {out}")
             return 0
-        print("gen_mc_tables: the reference's include/tables.h was not found (tried: "
-              + ", ".join(tried) + ") and no previously generated " + out + " exists; "
-              "pass its path as the first argument or set KF_MC_TABLES_H or KF_REFERENCE_DIR",
-              file=sys.stderr)
-        return 1
+        if len(argv) > 1:
+            print(f"gen_mc_tables: {argv[1]} was not found", file=sys.stderr)
+            return 1
+        emit(derive(), out)
+        print(f"gen_mc_tables: no tables.h found; derived {out} from the cube's geometry")
+        return 0
     emit(parse(src), out)
     print(f"gen_mc_tables: wrote {out}")
     return 0

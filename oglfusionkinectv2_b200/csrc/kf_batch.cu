@@ -262,6 +262,7 @@ void free_batch(kf_batch* b) {
   cudaFree(b->d_heads);
   cudaFreeHost(b->h_heads);
   cudaFree(b->d_inputs);
+  cudaFree(b->d_plan);
   cudaFreeHost(b->h_inputs);
   for (auto& row : b->ev)
     for (auto& e : row)
@@ -307,6 +308,10 @@ int kf_batch_create(int max_sessions, kf_batch** out) {
     return bail(KF_ERR_OUT_OF_MEMORY);
   if (cudaMalloc((void**)&b->d_inputs, max_sessions * sizeof(uint16_t*)) != cudaSuccess)
     return bail(KF_ERR_OUT_OF_MEMORY);
+  if (cudaMalloc((void**)&b->d_plan, (max_sessions + 1) * sizeof(unsigned)) != cudaSuccess)
+    return bail(KF_ERR_OUT_OF_MEMORY);
+  if (cudaMemsetAsync(b->d_plan, 0, (max_sessions + 1) * sizeof(unsigned), b->stream) != cudaSuccess)
+    return bail(KF_ERR_CUDA);
   *out = b;
   return KF_OK;
 }
@@ -377,7 +382,7 @@ int kf_batch_set_launch_shape(kf_batch* b, const kf_launch_shape* shape) {
   KF_CUDA_TRY(b, cudaStreamSynchronize(b->stream));
   b->int_zc = shape->integrate_z_chunk;
   b->ray_rows = shape->raycast_rows;
-  // the integrate block prefix depends on the z-chunk: rebuild the tables at the next step
+  drop_graphs(b);  // the captured steps hold the old shapes
   b->members.clear();
   b->member_keys.clear();
   return KF_OK;

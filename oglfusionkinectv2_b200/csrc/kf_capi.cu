@@ -62,6 +62,11 @@ int validate(const kf_config* c, const kf_intrinsics* in) {
   return KF_OK;
 }
 
+// 8x8 and 16x16 pixel tiles of a depth frame
+size_t tile_count(int w, int h) {
+  return (size_t)((w + 7) / 8) * ((h + 7) / 8) + (size_t)((w + 15) / 16) * ((h + 15) / 16);
+}
+
 size_t value_bytes(int storage) { return storage == KF_STORAGE_F32F32 ? 4 : 2; }
 
 void free_mc(kf_session* s) {
@@ -108,6 +113,8 @@ void free_all(kf_session* s) {
   free_mc(s);
   cudaFree(s->d_vol);
   cudaFree(s->d_bricks);
+  cudaFree(s->d_plan);
+  cudaFree(s->d_tiles);
   cudaFree(s->d_depth_u16);
   cudaFree(s->d_depth_f32_in);
   for (int l = 0; l < 3; ++l) {
@@ -210,6 +217,8 @@ int alloc_volume(kf_session* s) {
   s->d_vol = nullptr;
   cudaFree(s->d_bricks);
   s->d_bricks = s->d_supers = nullptr;
+  cudaFree(s->d_plan);
+  s->d_plan = nullptr;
   s->bx = (s->cfg.nx + KF_BRICK - 1) / KF_BRICK;
   s->by = (s->cfg.ny + KF_BRICK - 1) / KF_BRICK;
   s->bz = (s->cfg.nz + KF_BRICK - 1) / KF_BRICK;
@@ -222,6 +231,8 @@ int alloc_volume(kf_session* s) {
     if (rc) return rc;
     s->d_supers = s->d_bricks + nb;
     if ((rc = kf_reset_bricks(s))) return rc;
+    if ((rc = dalloc(s, &s->d_plan, KF_PLAN_HEAD + nb))) return rc;
+    KF_CUDA_TRY(s, cudaMemsetAsync(s->d_plan, 0, KF_PLAN_HEAD * 4, s->stream));
   }
   s->vol_count = (size_t)s->cfg.nx * s->cfg.ny * s->cfg.nz;
   s->vol_value_bytes = value_bytes(s->cfg.storage);
@@ -512,9 +523,10 @@ int kf_session_device_bytes(const kf_config* cfg, const kf_intrinsics* in, uint6
   const uint64_t px = (uint64_t)in->width * in->height;
   uint64_t b = vox * value_bytes(cfg->storage) * 2;
   b += (uint64_t)((cfg->nx + KF_BRICK - 1) / KF_BRICK) * ((cfg->ny + KF_BRICK - 1) / KF_BRICK) *
-       ((cfg->nz + KF_BRICK - 1) / KF_BRICK) * 4 +
+       ((cfg->nz + KF_BRICK - 1) / KF_BRICK) * 8 +
        (uint64_t)((cfg->nx + KF_SUPER - 1) / KF_SUPER) * ((cfg->ny + KF_SUPER - 1) / KF_SUPER) *
-       ((cfg->nz + KF_SUPER - 1) / KF_SUPER) * 4;  // brick and super-brick flags
+       ((cfg->nz + KF_SUPER - 1) / KF_SUPER) * 4;  // brick and super-brick flags, integrate's plan
+  b += KF_PLAN_HEAD * 4 + tile_count(in->width, in->height) * 4;
   b += px * (2 + 4) + px * 2 * kf_session::kRing;  // staging, and the frame graphs' inputs
   b += px * (4 + 16 + 16 + 4) * 2;         // three levels (sum < 4/3 of level 0)
   b += px * 32;                            // raycast maps
@@ -573,6 +585,8 @@ int kf_create(const kf_config* cfg, const kf_intrinsics* intr, kf_session** out)
     cudaMemsetAsync(s->d_normal[l], 0, n * 16, s->stream);
     cudaMemsetAsync(s->d_status[l], 0, n * 4, s->stream);
   }
+  if ((rc = dalloc(s, &s->d_tiles, tile_count(s->W[0], s->H[0])))) return bail(rc);
+  cudaMemsetAsync(s->d_tiles, 0, tile_count(s->W[0], s->H[0]) * 4, s->stream);
   if ((rc = dalloc(s, &s->d_ref_vertex, px))) return bail(rc);
   if ((rc = dalloc(s, &s->d_ref_normal, px))) return bail(rc);
   if ((rc = dalloc(s, &s->d_sdf_rows, px * 8))) return bail(rc);

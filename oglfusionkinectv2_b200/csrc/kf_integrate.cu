@@ -8,23 +8,22 @@
 // below 0.2, clamped to [-0.1, 0.2] with w = min(w + 1, maxWeight); otherwise (and for
 // eta <= -mu) value and weight are zeroed (Q8).
 //
-// B200 design: a block owns 32 x 8 columns by ZC z (one warp = 32 consecutive x: 64 B
-// per plane per z-step for 2-byte storage, fully used sectors); splitting the z-march
-// over ZC-voxel chunks (8, 16 or 32, tuned per volume) gives the SMs enough independent
-// warps to hide the depth-gather and volume latencies.  A block whose voxel box lies outside one of the five frustum
-// half-spaces returns at once, so voxels that cannot project into the image cost nothing;
-// inside, every voxel runs the reference's tests.  Per voxel one reciprocal replaces the
-// shader's divisions by z (u = fx * x/z + cx + 0.5 is the reference's (fx x + cx z)/z + 0.5
-// up to rounding), and the reciprocal, square root and running-average division use the
-// hardware approximations (2 ulp; GLSL allows 2.5 ulp for division).  The weight plane is read only where eta > -mu, and a voxel whose
-// encoded value and weight do not change is not written back.
+// B200 design: two launches.  The plan kernel tests every 8^3 brick, one thread each, and
+// lists the bricks the frame can change; the integrate kernel runs the reference's tests on
+// the voxels of the listed bricks only.  Of the voxels that project into the image about six
+// in ten lie more than mu behind the surface (rewritten with zero, which changes nothing in
+// a brick that holds only zeros) and three in ten see a zero depth pixel (skipped), so most
+// bricks drop out on the farthest depth of the tiles their projection covers.
+// What bounds it: instruction issue and the L1 request rate, not DRAM (194 MB read and 64 MB
+// written for 63 M listed voxels of a 768^3 room frame).  Integrate at 512^3 F16U16 (both
+// launches): 181 -> 50 us, at 768^3 427 -> 206 us, 16 batched sessions 917 -> 412 us.
 #include "kf_internal.cuh"
 
 namespace {
 
 struct IntArgs {
   void* vol;
-  size_t count;
+  size_t count_voxels;
   int nx, ny, nz;
   float dimx, dimy, dimz;
   const float* depth;
@@ -38,6 +37,12 @@ struct IntArgs {
   int bx, by, bz;
   uint32_t* supers;
   int sbx, sby, sbz;
+  // the farthest depths of 8x8 and 16x16 pixel tiles (kf_pyramid.cu)
+  const float* tiles8;
+  const float* tiles16;
+  int tw8, tw16;
+  uint32_t* list;   // planned bricks
+  unsigned* count;  // their number (zero between launches)
 };
 
 template <class T>
@@ -46,10 +51,6 @@ __device__ __forceinline__ uint32_t bits_of(const T& v) {
   memcpy(&b, &v, sizeof(T));
   return b;
 }
-
-// Voxels per thread along z (the block's brick of columns is 32 x 8 x ZC): one of
-// KF_INT_ZCHUNKS, chosen per session (default 16, or the autotuner's pick).  Every choice
-// computes the same volume.
 
 // True when the box of voxel centres [b0, b1] (index space, inclusive) lies entirely on the
 // outside of one of the five half-spaces whose intersection is the set of voxels
@@ -76,61 +77,244 @@ __device__ __forceinline__ bool box_outside_frustum(const IntArgs& a, const floa
          (o3 & 0xffu) == 0xffu || (o4 & 0xffu) == 0xffu;
 }
 
-// The z-chunk [zb, zb + ZC) of column (x, y); returns which z-bricks received a negative
-// value (bit j = brick zb/8 - 1 + j, bit 0 for the dilation of a z % 8 == 0 voxel).
-template <int S, int ZC>
-__device__ __forceinline__ uint32_t integrate_column(const IntArgs& a, const float* inv, int x, int y, int zb) {
+// A batched launch: plan block b belongs to the entry e with prefix[e] <= b < prefix[e + 1];
+// the integrate kernel walks all entries' lists (counts[e] bricks each) as one.
+struct IntBatch {
+  const IntArgs* args;
+  const uint32_t* prefix;  // n + 1 entries
+  unsigned* counts;        // n counts
+  unsigned* done;          // blocks of the integrate launch that are through (zero between launches)
+  int n;
+};
+
+// A plan block covers 8 x 8 x 4 bricks; list entries hold the brick's coordinates (at most
+// 512 per axis) and whether it held anything but zeros.
+constexpr int kPlanX = 8, kPlanY = 8, kPlanZ = 4;
+constexpr uint32_t kEntrySet = 1u << 27;
+__device__ __forceinline__ uint32_t entry_of(int bx, int by, int bz) {
+  return (uint32_t)bx | (uint32_t)by << 9 | (uint32_t)bz << 18;
+}
+
+// Whether integrate.cs may change a voxel of brick (bx, by, bz), whose flag word is `word`.
+// False only when no voxel of it can: the brick (grown by half a voxel on every side, which
+// also covers the rounding of the per-voxel positions) lies outside the view frustum, or on
+// every depth pixel that its projection may touch the voxels are skipped (depth 0) or, in a
+// brick that holds only zeros, zeroed (d - z <= -mu).  The ray-length factor is >= 1, so
+// d - z <= -mu, with a margin for rounding, implies eta <= -mu.
+__device__ __forceinline__ bool brick_changes(const IntArgs& a, const float* inv, int bx, int by, int bz,
+                                              uint32_t word) {
+  const float vx = a.dimx / a.nx, vy = a.dimy / a.ny, vz = a.dimz / a.nz;
+  const float wx = (float)(bx * KF_BRICK) * vx, wy = (float)(by * KF_BRICK) * vy, wz = (float)(bz * KF_BRICK) * vz;
+  const float ex = (float)min(KF_BRICK, a.nx - bx * KF_BRICK) * vx, ey = (float)min(KF_BRICK, a.ny - by * KF_BRICK) * vy,
+              ez = (float)min(KF_BRICK, a.nz - bz * KF_BRICK) * vz;
+  float o[3], ax[3], ay[3], az[3], mag = 0.0f;  // the low corner and the three edges in camera space
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    o[r] = inv[r * 4] * wx + inv[r * 4 + 1] * wy + inv[r * 4 + 2] * wz + inv[r * 4 + 3];
+    ax[r] = inv[r * 4] * ex;
+    ay[r] = inv[r * 4 + 1] * ey;
+    az[r] = inv[r * 4 + 2] * ez;
+    mag = fmaxf(mag, fabsf(inv[r * 4]) * a.dimx + fabsf(inv[r * 4 + 1]) * a.dimy + fabsf(inv[r * 4 + 2]) * a.dimz +
+                         fabsf(inv[r * 4 + 3]));
+  }
+  if (!(mag < 1e30f)) return true;
+  // outside one of the five half-spaces: the largest value over the corners is negative
+  auto top = [&](float kx, float ky, float kz) {
+    return kx * o[0] + ky * o[1] + kz * o[2] + fmaxf(0.0f, kx * ax[0] + ky * ax[1] + kz * ax[2]) +
+           fmaxf(0.0f, kx * ay[0] + ky * ay[1] + kz * ay[2]) + fmaxf(0.0f, kx * az[0] + ky * az[1] + kz * az[2]);
+  };
+  const float ku = a.cx + 0.5f, kv = a.cy + 0.5f;
+  const float W1 = (float)(a.W - 1), H1 = (float)(a.H - 1);
+  if (top(0.0f, 0.0f, 1.0f) < 1e-4f || top(a.fx, 0.0f, ku) < 0.0f || top(-a.fx, 0.0f, W1 - ku) < 0.0f ||
+      top(0.0f, a.fy, kv) < 0.0f || top(0.0f, -a.fy, H1 - kv) < 0.0f)
+    return false;
+  const float zmin = o[2] + fminf(0.0f, ax[2]) + fminf(0.0f, ay[2]) + fminf(0.0f, az[2]);
+  if (!(zmin > 0.01f)) return true;  // reaches the camera plane: no bounded projection
+  // the pixels it may touch: the bounding box of the corners' projections (every corner is in
+  // front of the camera), a pixel and the positions' rounding wider
+  float u0 = 1e30f, u1 = -1e30f, v0 = 1e30f, v1 = -1e30f;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float X = o[0] + (c & 1 ? ax[0] : 0.0f) + (c & 2 ? ay[0] : 0.0f) + (c & 4 ? az[0] : 0.0f);
+    const float Y = o[1] + (c & 1 ? ax[1] : 0.0f) + (c & 2 ? ay[1] : 0.0f) + (c & 4 ? az[1] : 0.0f);
+    const float Z = o[2] + (c & 1 ? ax[2] : 0.0f) + (c & 2 ? ay[2] : 0.0f) + (c & 4 ? az[2] : 0.0f);
+    const float iz = __fdividef(1.0f, Z);
+    const float u = fmaf(a.fx, X * iz, ku), v = fmaf(a.fy, Y * iz, kv);
+    u0 = fminf(u0, u);
+    u1 = fmaxf(u1, u);
+    v0 = fminf(v0, v);
+    v1 = fmaxf(v1, v);
+  }
+  const float slack = 4e-6f * mag;
+  const float m = 1.0f + slack * fmaxf(a.fx, a.fy) * __fdividef(1.0f, zmin);
+  u0 = fmaxf(u0 - m, 0.0f);
+  v0 = fmaxf(v0 - m, 0.0f);
+  u1 = fminf(u1 + m, W1);
+  v1 = fminf(v1 + m, H1);
+  if (u0 > u1 || v0 > v1) return false;
+  const float reach = word & KF_BRICK_SET ? -INFINITY : zmin - a.mu - 1e-4f * (zmin + a.mu) - slack;
+  const int x0 = (int)u0, x1 = (int)u1, y0 = (int)v0, y1 = (int)v1;
+  // tiles of the finest level that covers the box in few reads; a box too wide for that is
+  // a brick close to the camera
+  int sh = 3, tw = a.tw8;
+  const float* t = a.tiles8;
+  if (((x1 >> 3) - (x0 >> 3) + 1) * ((y1 >> 3) - (y0 >> 3) + 1) > 16) {
+    sh = 4;
+    tw = a.tw16;
+    t = a.tiles16;
+    if (((x1 >> 4) - (x0 >> 4) + 1) * ((y1 >> 4) - (y0 >> 4) + 1) > 100) return true;
+  }
+  // no early exit: the loads do not wait for one another
+  float far = -INFINITY;
+  for (int ty = y0 >> sh; ty <= y1 >> sh; ++ty)
+#pragma unroll 4
+    for (int tx = x0 >> sh; tx <= x1 >> sh; ++tx) far = fmaxf(far, __ldg(t + ty * tw + tx));
+  return far * 0.001f > reach;
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(256) plan_kernel(IntArgs one, IntBatch batch) {
+  __shared__ unsigned s_n[9];
+  int local = blockIdx.x, e = 0;
+  if constexpr (BATCH) {
+    // binary search of the entry (uniform over the block)
+    int lo = 0, hi = batch.n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(batch.prefix + mid) <= blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    e = lo;
+    local = (int)(blockIdx.x - __ldg(batch.prefix + e));
+  }
+  const IntArgs& a = BATCH ? batch.args[e] : one;
+  if (a.gate && *(volatile const int*)a.gate == 0) return;
+  float inv[12];  // inverse(m_pose), rows of [R^T | -R^T t] (integrate uses glm::inverse, :1242)
+#pragma unroll
+  for (int k = 0; k < 12; ++k) inv[k] = a.st->inv_rows[k];
+  const int gx = (a.bx + kPlanX - 1) / kPlanX, gy = (a.by + kPlanY - 1) / kPlanY;
+  const int x0 = local % gx * kPlanX, y0 = local / gx % gy * kPlanY, z0 = local / (gx * gy) * kPlanZ;
+  // the whole block's box first (every warp finds the same answer); one voxel of margin
+  {
+    const int b0[3] = {x0 * KF_BRICK - 1, y0 * KF_BRICK - 1, z0 * KF_BRICK - 1};
+    const int b1[3] = {(x0 + kPlanX) * KF_BRICK, (y0 + kPlanY) * KF_BRICK, (z0 + kPlanZ) * KF_BRICK};
+    if (box_outside_frustum(a, inv, b0, b1)) return;
+  }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bx = x0 + (tid & 7), by = y0 + ((tid >> 3) & 7), bz = z0 + (tid >> 6);
+  bool work = false;
+  uint32_t word = 0;
+  if (bx < a.bx && by < a.by && bz < a.bz) {
+    word = a.bricks[(uint32_t)bx + (uint32_t)a.bx * ((uint32_t)by + (uint32_t)a.by * (uint32_t)bz)];
+    work = brick_changes(a, inv, bx, by, bz, word);
+  }
+  const unsigned mine = __ballot_sync(0xffffffffu, work);
+  if (lane == 0) s_n[warp] = __popc(mine);
+  __syncthreads();
+  if (tid == 0) {
+    unsigned n = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const unsigned c = s_n[w];
+      s_n[w] = n;
+      n += c;
+    }
+    s_n[8] = n ? atomicAdd(a.count, n) : 0u;
+  }
+  __syncthreads();
+  if (work)
+    a.list[s_n[8] + s_n[warp] + __popc(mine & ((1u << lane) - 1u))] =
+        entry_of(bx, by, bz) | (word & KF_BRICK_SET ? kEntrySet : 0u);
+}
+
+// Hardware reciprocal and reciprocal square root of normal numbers: the values of __fdividef
+// and rsqrtf without their scaling of denormals, which no operand here is.
+__device__ __forceinline__ float mufu_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float mufu_rsqrt(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Half of a listed brick by one warp: lane = (x, y) column (8 x 4 of them), its 8 voxels
+// along z in registers.  The loads of a step (depth pixels, then values and weights) are
+// issued for all 8 voxels together: a column waits for two memory latencies, not sixteen.
+// 64 registers, no spills: a variant with fewer instructions (border tests left out for inner
+// bricks, the ray length only near the surface) spilled and was slower.
+template <int S>
+__device__ __forceinline__ void integrate_half_brick(const IntArgs& a, uint32_t entry, int half, int lane) {
   typedef typename Vox<S>::V V;
   typedef typename Vox<S>::Wt Wt;
-  // bits 0..ZC/8: NEG of z-bricks zb/8 - 1 + j; bit 6: NEG of z-super-brick zb/64, bit 7:
-  // of zb/64 - 1 (a z % 64 == 0 voxel is that one's +1 layer)
-  static_assert(ZC == 8 || ZC == 16 || ZC == 32, "z chunk: 8, 16 or 32 voxels");
-  uint32_t flags = 0;
+  const int bx = entry & 511, by = (entry >> 9) & 511, bz = (entry >> 18) & 511;
+  const int x = bx * KF_BRICK + (lane & 7), y = by * KF_BRICK + 4 * half + (lane >> 3), z0 = bz * KF_BRICK;
+  const bool was_set = (entry & kEntrySet) != 0;
+  const int zend = (x < a.nx && y < a.ny) ? min(KF_BRICK, a.nz - z0) : 0;
 
   // getVolumePosition (integrate.cs:16-19; along z as (i + 0.5) * voxel size) and
   // delta = rotate(invTrack, (0,0,vz)): the camera-space position is computed directly at
-  // every z % 8 == 0 voxel and stepped by delta in between, so it does not depend on where
-  // a chunk starts (every z-chunk size gives the same volume)
+  // the brick's first voxel and steps by delta inside it (:57-62)
   const float cxw = (x + 0.5f) * a.dimx / a.nx;
   const float cyw = (y + 0.5f) * a.dimy / a.ny;
   const float vz = a.dimz / a.nz;
-  float pxy[3], dz[3];
+  const float czw = (z0 + 0.5f) * vz;
+  const float* inv = a.st->inv_rows;  // inverse(m_pose), rows of [R^T | -R^T t] (glm::inverse, :1242)
+  float pos[3], dz[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    pxy[r] = fmaf(inv[r * 4 + 0], cxw, fmaf(inv[r * 4 + 1], cyw, inv[r * 4 + 3]));
+    pos[r] = fmaf(inv[r * 4 + 2], czw, fmaf(inv[r * 4 + 0], cxw, fmaf(inv[r * 4 + 1], cyw, inv[r * 4 + 3])));
     dz[r] = __fmul_rn(inv[r * 4 + 2], vz);  // kept rounded: the steps below are plain adds
   }
-  V* vf = reinterpret_cast<V*>(a.vol);
-  Wt* vw = reinterpret_cast<Wt*>(reinterpret_cast<char*>(a.vol) + a.count * sizeof(V));
-  const uint32_t slice = (uint32_t)a.nx * (uint32_t)a.ny;
-  uint32_t idx = (uint32_t)x + (uint32_t)a.nx * (uint32_t)y + (uint32_t)zb * slice;
   const float fW1 = (float)(a.W - 1), fH1 = (float)(a.H - 1);
   const float ku = a.cx + 0.5f, kv = a.cy + 0.5f;
-  const int zend = min(ZC, a.nz - zb);
-  float px, py, pz;
-  // one voxel of the march (integrate.cs:63-113); jj: its index in the current brick
-  auto voxel = [&](int jj, int jb, int k8) {
-    if (pz < 0.0001f) return;
-    const float iz = __fdividef(1.0f, pz);  // hardware reciprocal (2 ulp)
+  float pz[8], len[8], d[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    d[j] = 0.0f;
+    const float px = pos[0], py = pos[1];
+    pz[j] = pos[2];
+    const float iz = mufu_rcp(pz[j]);  // 2 ulp
     const float rx = px * iz;  // pos.x / pos.z
     const float ry = py * iz;
     // cameraX.x / cameraX.z + 0.5 = fx * x/z + cx + 0.5 (K has no skew, :67)
     const float u = fmaf(a.fx, rx, ku);
     const float v = fmaf(a.fy, ry, kv);
-    if (u < 0.0f || u > fW1 || v < 0.0f || v > fH1) return;
-    // explicitly rounded: no template instance may fuse the scaling into the subtraction,
-    // so every launch shape computes the same bits
-    const float d = __fmul_rn(__ldg(a.depth + (uint32_t)(int)v * (uint32_t)a.W + (uint32_t)(int)u), 0.001f);
-    if (d == 0.0f) return;
     const float r2 = fmaf(rx, rx, fmaf(ry, ry, 1.0f));
-    const float diff = __fmul_rn(__fsub_rn(d, pz), __fmul_rn(r2, rsqrtf(r2)));  // sqrt(r2), r2 >= 1
-    if (diff > -a.mu) {
-      const float sdf = fminf(1.0f, __fmul_rn(diff, a.inv_mu));
-      const V oldv = vf[idx];
-      const Wt oldw = vw[idx];
-      const float F = __fmul_rn(Vox<S>::raw_nc(&oldv, 0), Vox<S>::kRawToF);
-      const float w = Vox<S>::weight(&oldw, 0);
-      const float wd = __fdividef(fmaf(w, F, sdf), w + 1.0f);
+    len[j] = __fmul_rn(r2, mufu_rsqrt(r2));  // sqrt(r2), r2 >= 1
+    const bool out = pz[j] < 0.0001f || u < 0.0f || u > fW1 || v < 0.0f || v > fH1;
+    if (j < zend && !out) d[j] = __ldg(a.depth + kf_trunc_index(v, u, (uint32_t)a.W));
+#pragma unroll
+    for (int r = 0; r < 3; ++r) pos[r] += dz[r];
+  }
+  V* vf = reinterpret_cast<V*>(a.vol);
+  Wt* vw = reinterpret_cast<Wt*>(reinterpret_cast<char*>(a.vol) + a.count_voxels * sizeof(V));
+  const uint32_t slice = (uint32_t)a.nx * (uint32_t)a.ny;
+  const uint32_t idx0 = (uint32_t)x + (uint32_t)a.nx * (uint32_t)y + (uint32_t)z0 * slice;
+  V oldv[8];
+  Wt oldw[8];
+  uint32_t fuse = 0, hit = 0;  // bit j: voxel j is averaged; sees a depth
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float dm = __fmul_rn(d[j], 0.001f);
+    if (dm != 0.0f) hit |= 1u << j;
+    // explicitly rounded: no launch fuses the scaling into the subtraction
+    d[j] = __fmul_rn(__fsub_rn(dm, pz[j]), len[j]);
+    if (dm != 0.0f && d[j] > -a.mu) {
+      fuse |= 1u << j;
+      oldv[j] = vf[idx0 + j * slice];
+      oldw[j] = vw[idx0 + j * slice];
+    }
+  }
+  bool set = false, neg = false, neg0 = false;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (fuse >> j & 1u) {
+      const float sdf = fminf(1.0f, __fmul_rn(d[j], a.inv_mu));
+      const float F = __fmul_rn(Vox<S>::raw_nc(&oldv[j], 0), Vox<S>::kRawToF);
+      const float w = Vox<S>::weight(&oldw[j], 0);
+      const float wd = fmaf(w, F, sdf) * mufu_rcp(w + 1.0f);
       float nF, nw;
       if (!a.band) {
         // the reference's earlier update (integrate.cs:115-150)
@@ -145,134 +329,113 @@ __device__ __forceinline__ uint32_t integrate_column(const IntArgs& a, const flo
       }
       const V ev = Vox<S>::encode_value(nF);
       const Wt ew = Vox<S>::encode_weight(nw);
-      if (bits_of(ev) != bits_of(oldv)) vf[idx] = ev;
-      if (bits_of(ew) != bits_of(oldw)) vw[idx] = ew;
-      // a non-negative nF never stores a negative value; a brick's first voxel is also
-      // the +1 layer of the brick below it (and, at z % 64 == 0, of the super-brick below)
-      if (nF < 0.0f) {
-        flags |= 1u << jb;
-        if (jj == 0) flags |= (1u << (jb - 1)) | (((zb + k8) & 63) == 0 ? 0xc0u : 0x40u);
-        else flags |= 0x40u;
+      if (bits_of(ev) != bits_of(oldv[j])) vf[idx0 + j * slice] = ev;
+      if (bits_of(ew) != bits_of(oldw[j])) vw[idx0 + j * slice] = ew;
+      set |= (bits_of(ev) | bits_of(ew)) != 0;
+      // a non-negative nF never stores a negative value
+      neg |= nF < 0.0f;
+      if (j == 0) neg0 = nF < 0.0f;
+    }
+  }
+  if (was_set && __any_sync(0xffffffffu, (hit & ~fuse) != 0)) {
+    // eta <= -mu: zeroed (already zero in a brick that held only zeros)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if ((hit & ~fuse) >> j & 1u) {
+        vf[idx0 + j * slice] = Vox<S>::encode_value(0.0f);
+        vw[idx0 + j * slice] = Vox<S>::encode_weight(0.0f);
       }
-    } else {
-      vf[idx] = Vox<S>::encode_value(0.0f);
-      vw[idx] = Vox<S>::encode_weight(0.0f);
-    }
-  };
-  // One 8-voxel brick of the column at a time: the position is anchored at the brick's first
-  // voxel and steps by delta inside it, as integrate.cs:57-62 does, so it does not depend on
-  // where a chunk starts.  Whole bricks run unrolled; only a ragged last brick (nz not a
-  // multiple of 8) takes the counted loop.
-  for (int k8 = 0; k8 < zend; k8 += 8) {
-    const float czw = (zb + k8 + 0.5f) * vz;
-    px = fmaf(inv[2], czw, pxy[0]);
-    py = fmaf(inv[6], czw, pxy[1]);
-    pz = fmaf(inv[10], czw, pxy[2]);
-    const int jb = (k8 >> 3) + 1;  // this brick's bit in flags
-    if (k8 + 8 <= zend) {
-#pragma unroll
-      for (int jj = 0; jj < 8; ++jj, idx += slice, px += dz[0], py += dz[1], pz += dz[2]) voxel(jj, jb, k8);
-    } else {
-      for (int jj = 0; jj < zend - k8; ++jj, idx += slice, px += dz[0], py += dz[1], pz += dz[2]) voxel(jj, jb, k8);
-    }
   }
-  return flags;
-}
-
-// A batched launch: flat block b belongs to the entry e with prefix[e] <= b < prefix[e + 1].
-struct IntBatch {
-  const IntArgs* args;
-  const uint32_t* prefix;  // n + 1 entries
-  int n;
-};
-
-template <int S, bool BATCH, int ZC>
-__global__ void __launch_bounds__(256, 6) integrate_kernel(IntArgs a_one, IntBatch batch) {
-  __shared__ IntArgs s_args;
-  int bxi, byi, bzi;  // this block's position in its volume's block grid
-  if constexpr (BATCH) {
-    // binary search of the entry (uniform over the block)
-    int lo = 0, hi = batch.n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(batch.prefix + mid) <= blockIdx.x) lo = mid; else hi = mid - 1;
-    }
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const int* src = reinterpret_cast<const int*>(batch.args + lo);
-    for (int k = tid; k < (int)(sizeof(IntArgs) / 4); k += 256) reinterpret_cast<int*>(&s_args)[k] = __ldg(src + k);
-    __syncthreads();
-    const uint32_t local = blockIdx.x - __ldg(batch.prefix + lo);
-    const uint32_t gx = (uint32_t)(s_args.nx + 31) / 32, gy = (uint32_t)(s_args.ny + 7) / 8;
-    bxi = (int)(local % gx);
-    byi = (int)((local / gx) % gy);
-    bzi = (int)(local / (gx * gy));
-  } else {
-    bxi = blockIdx.x;
-    byi = blockIdx.y;
-    bzi = blockIdx.z;
-  }
-  const IntArgs& a = BATCH ? s_args : a_one;
-  if (a.gate && *(volatile const int*)a.gate == 0) return;
-  float inv[12];  // inverse(m_pose), rows of [R^T | -R^T t] (integrate uses glm::inverse, :1242)
-#pragma unroll
-  for (int k = 0; k < 12; ++k) inv[k] = a.st->inv_rows[k];
-  const int xb = bxi * 32, yb = byi * 8, zb = bzi * ZC;
-  // Every warp evaluates the block's frustum test itself (the same inputs give the same
-  // answer in every warp), so no warp waits for another: the kernel has no block barrier.
-  // One voxel of margin on every side absorbs the rounding of the per-voxel tests.
-  {
-    const int b0[3] = {xb - 1, yb - 1, zb - 1};
-    const int b1[3] = {xb + 32, yb + 8, zb + ZC};
-    if (box_outside_frustum(a, inv, b0, b1)) return;
-  }
-  const int lane = threadIdx.x;
-  const int x = xb + lane;
-  const int y = yb + threadIdx.y;  // uniform over the warp
-  uint32_t flags = 0;  // integrate_column's bits
-  if (x < a.nx && y < a.ny) flags = integrate_column<S, ZC>(a, inv, x, y, zb);
-  if (!__any_sync(0xffffffffu, flags != 0)) return;
-  // Brick flags, merged over the warp: lanes 8c-8..8c-1 write brick column c of the block
-  // (c = 1..4) and a lane on a brick's low x face also brick column c-1 (dilation); lane c
-  // sets the merged bits of column c in global memory.  Most bricks near surfaces have the
-  // bits already, so read first and skip those atomics.
-  const int lx = (x >> 3) - (xb >> 3) + 1;
-  constexpr int kZBits = ZC / 8 + 1;  // z-bricks a chunk touches, with the dilation one
-  const uint32_t zbits = flags & ((1u << kZBits) - 1u);
-  uint32_t mine = 0;
-#pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    const uint32_t m = (lx == c ? zbits : 0u) | (lx - 1 == c && (x & 7) == 0 ? zbits : 0u);
-    const uint32_t r = __reduce_or_sync(0xffffffffu, m);
-    if (lane == c) mine = r;
-  }
-  if (lane < 5 && mine) {
-    const int gx = (xb >> 3) - 1 + lane;
-    for (int j = 0; j < kZBits; ++j) {
-      if (!((mine >> j) & 1u)) continue;
-      const int gz = (zb >> 3) - 1 + j;
-      for (int dy = 0; dy < ((y & 7) == 0 ? 2 : 1); ++dy) {
-        const int gy = (y >> 3) - dy;
-        if (gx >= 0 && gy >= 0 && gz >= 0 && gx < a.bx && gy < a.by && gz < a.bz) {
-          uint32_t* w = &a.bricks[(uint32_t)gx + (uint32_t)a.bx * ((uint32_t)gy + (uint32_t)a.by * (uint32_t)gz)];
-          if (!(*(volatile uint32_t*)w & KF_BRICK_NEG)) atomicOr(w, KF_BRICK_NEG);
-        }
-      }
-    }
-  }
-  // super-bricks: own and, on a super-brick's low face, the one below (x, y, z)
-  const uint32_t sbits = flags & 0xc0u;
-  const uint32_t s_own = __reduce_or_sync(0xffffffffu, sbits);
-  const uint32_t s_lowx = __reduce_or_sync(0xffffffffu, (x & 63) == 0 ? sbits : 0u);
-  if (lane < 8 && (lane & 1 ? s_own : s_lowx)) {
-    const int jx = lane & 1, jy = (lane >> 1) & 1, jz = lane >> 2;
-    const uint32_t zsel = jz ? 0x40u : 0x80u;
-    const uint32_t src = jx ? s_own : s_lowx;
-    if ((src & zsel) && (jy == 1 || (y & 63) == 0)) {
-      const int gx = (xb >> 6) - 1 + jx, gy = (y >> 6) - 1 + jy, gz = (zb >> 6) - 1 + jz;
-      if (gx >= 0 && gy >= 0 && gz >= 0 && gx < a.sbx && gy < a.sby && gz < a.sbz) {
-        uint32_t* w = &a.supers[(uint32_t)gx + (uint32_t)a.sbx * ((uint32_t)gy + (uint32_t)a.sby * (uint32_t)gz)];
+  // Brick flags: lane c merges corner c of the dilation (a brick's low x, y or z layer is
+  // also the +1 layer of the brick below it) and sets the brick's and its super-brick's bit
+  // where it is still clear.
+  const unsigned b_set = __ballot_sync(0xffffffffu, set), b_neg = __ballot_sync(0xffffffffu, neg),
+                 b_neg0 = __ballot_sync(0xffffffffu, neg0);
+  if (lane < 8 && (b_set | b_neg)) {
+    const int gx = bx - (lane & 1), gy = by - ((lane >> 1) & 1), gz = bz - (lane >> 2);
+    unsigned m = lane & 4 ? b_neg0 : b_neg;
+    if (lane & 1) m &= 0x01010101u;
+    if (lane & 2) m &= half ? 0u : 0xffu;
+    uint32_t want = m ? KF_BRICK_NEG : 0u;
+    if (lane == 0 && b_set) want |= KF_BRICK_SET;
+    if (want && gx >= 0 && gy >= 0 && gz >= 0) {
+      uint32_t* w = &a.bricks[(uint32_t)gx + (uint32_t)a.bx * ((uint32_t)gy + (uint32_t)a.by * (uint32_t)gz)];
+      if (want & ~*(volatile uint32_t*)w) atomicOr(w, want);
+      if (want & KF_BRICK_NEG) {
+        w = &a.supers[(uint32_t)(gx >> 3) + (uint32_t)a.sbx * ((uint32_t)(gy >> 3) + (uint32_t)a.sby * (uint32_t)(gz >> 3))];
         if (!(*(volatile uint32_t*)w & KF_BRICK_NEG)) atomicOr(w, KF_BRICK_NEG);
       }
+    }
+  }
+}
+
+// Small volumes: every warp tests one brick and runs it at once, which saves the list and a
+// launch.  A warp's test costs about as many instructions as half a brick's voxels, all lanes
+// doing the same, so it pays only while the launches' latency dominates (see kSmallBricks).
+template <int S>
+__global__ void __launch_bounds__(256, 4) integrate_small_kernel(IntArgs a) {
+  if (a.gate && *(volatile const int*)a.gate == 0) return;
+  const int lane = threadIdx.x & 31, b = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (b >= a.bx * a.by * a.bz) return;
+  const int bx = b % a.bx, by = b / a.bx % a.by, bz = b / (a.bx * a.by);
+  const uint32_t word = a.bricks[b];
+  if (!brick_changes(a, a.st->inv_rows, bx, by, bz, word)) return;
+  const uint32_t entry = entry_of(bx, by, bz) | (word & KF_BRICK_SET ? kEntrySet : 0u);
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) integrate_half_brick<S>(a, entry, half, lane);
+}
+
+// Persistent: every warp takes `chunk` half-bricks of the list(s) per step until they are
+// through; the last block zeroes the counts for the next plan.
+template <int S, bool BATCH>
+__global__ void __launch_bounds__(256, 4) integrate_kernel(IntArgs one, IntBatch batch, int chunk) {
+  __shared__ uint32_t s_first[BATCH ? 257 : 1];  // first half-brick of each entry
+  __shared__ uint32_t s_warp[BATCH ? 8 : 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t total;
+  if constexpr (BATCH) {
+    const uint32_t c = tid < batch.n ? 2u * *(volatile const unsigned*)(batch.counts + tid) : 0u;
+    uint32_t inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) inc += s_warp[w];
+    s_first[tid] = inc - c;
+    if (tid == 255) s_first[256] = inc;
+    __syncthreads();
+    total = s_first[256];
+  } else {
+    total = 2u * *(volatile const unsigned*)one.count;
+  }
+  const uint32_t step = gridDim.x * 8u * (uint32_t)chunk;
+  for (uint32_t t0 = (blockIdx.x * 8u + warp) * (uint32_t)chunk; t0 < total; t0 += step)
+    for (uint32_t t = t0; t < min(t0 + (uint32_t)chunk, total); ++t) {
+      if constexpr (BATCH) {
+        int lo = 0, hi = batch.n - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (s_first[mid] <= t) lo = mid; else hi = mid - 1;
+        }
+        const uint32_t k = t - s_first[lo];
+        integrate_half_brick<S>(batch.args[lo], batch.args[lo].list[k >> 1], (int)(k & 1u), lane);
+      } else {
+        integrate_half_brick<S>(one, one.list[t >> 1], (int)(t & 1u), lane);
+      }
+    }
+  __syncthreads();  // every warp of the block has read the counts
+  if (tid == 0) {
+    unsigned* done = BATCH ? batch.done : one.count + 1;
+    if (atomicAdd(done, 1u) == gridDim.x - 1) {
+      if constexpr (BATCH) {
+        for (int e = 0; e < batch.n; ++e) batch.counts[e] = 0u;
+      } else {
+        *one.count = 0u;
+      }
+      *done = 0u;
     }
   }
 }
@@ -284,7 +447,7 @@ namespace {
 IntArgs make_int_args(kf_session* s, int gated) {
   IntArgs a;
   a.vol = s->d_vol;
-  a.count = s->vol_count;
+  a.count_voxels = s->vol_count;
   a.nx = s->cfg.nx; a.ny = s->cfg.ny; a.nz = s->cfg.nz;
   a.dimx = s->cfg.dim_x; a.dimy = s->cfg.dim_y; a.dimz = s->cfg.dim_z;
   a.depth = s->d_depth[0];
@@ -300,24 +463,49 @@ IntArgs make_int_args(kf_session* s, int gated) {
   a.bx = s->bx; a.by = s->by; a.bz = s->bz;
   a.supers = s->d_supers;
   a.sbx = s->sbx; a.sby = s->sby; a.sbz = s->sbz;
+  a.tiles8 = s->d_tiles;
+  a.tw8 = (a.W + 7) / 8;
+  a.tiles16 = s->d_tiles + (size_t)a.tw8 * ((a.H + 7) / 8);
+  a.tw16 = (a.W + 15) / 16;
+  a.count = s->d_plan;
+  a.list = s->d_plan + KF_PLAN_HEAD;
   return a;
 }
 
-template <bool BATCH, int ZC>
-void launch_int_zc(int storage, dim3 grid, cudaStream_t st, const IntArgs& a, const IntBatch& b) {
-  dim3 block(32, 8);
-  switch (storage) {
-    case KF_STORAGE_F32F32: integrate_kernel<KF_STORAGE_F32F32, BATCH, ZC><<<grid, block, 0, st>>>(a, b); break;
-    case KF_STORAGE_F16U16: integrate_kernel<KF_STORAGE_F16U16, BATCH, ZC><<<grid, block, 0, st>>>(a, b); break;
-    default: integrate_kernel<KF_STORAGE_RG16I, BATCH, ZC><<<grid, block, 0, st>>>(a, b); break;
-  }
+uint32_t plan_blocks(const IntArgs& a) {
+  return (uint32_t)((a.bx + kPlanX - 1) / kPlanX) * ((a.by + kPlanY - 1) / kPlanY) * ((a.bz + kPlanZ - 1) / kPlanZ);
 }
 
+// Volumes of at most this many bricks take the one-launch form.  Per call, one launch against
+// two (B200, back to back, events included): 64^3 18.5 / 27.2 us, 128^3 21.5 / 26.8, 160^3
+// 26.4 / 29.4, 192^3 33.0 / 31.3, 256^3 53 / 41.  The line lies between 160^3 and 192^3.
+constexpr int kSmallBricks = 8192;
+
+int brick_count(const IntArgs& a) { return a.bx * a.by * a.bz; }
+
+cudaError_t launch_int_small(int storage, cudaStream_t st, const IntArgs& a) {
+  const int grid = (brick_count(a) + 7) / 8;
+  switch (storage) {
+    case KF_STORAGE_F32F32: integrate_small_kernel<KF_STORAGE_F32F32><<<grid, 256, 0, st>>>(a); break;
+    case KF_STORAGE_F16U16: integrate_small_kernel<KF_STORAGE_F16U16><<<grid, 256, 0, st>>>(a); break;
+    default: integrate_small_kernel<KF_STORAGE_RG16I><<<grid, 256, 0, st>>>(a); break;
+  }
+  return cudaGetLastError();
+}
+
+// Four blocks of 256 threads per SM (the register budget), one wave.
 template <bool BATCH>
-void launch_int(int storage, int zc, dim3 grid, cudaStream_t st, const IntArgs& a, const IntBatch& b) {
-  if (zc == 8) launch_int_zc<BATCH, 8>(storage, grid, st, a, b);
-  else if (zc == 32) launch_int_zc<BATCH, 32>(storage, grid, st, a, b);
-  else launch_int_zc<BATCH, 16>(storage, grid, st, a, b);
+cudaError_t launch_int(int storage, int num_sms, uint32_t plan, int zc, cudaStream_t st, const IntArgs& a,
+                       const IntBatch& b) {
+  plan_kernel<BATCH><<<plan, 256, 0, st>>>(a, b);
+  if (cudaError_t e = cudaGetLastError()) return e;
+  const int grid = 4 * num_sms, chunk = zc / KF_BRICK;
+  switch (storage) {
+    case KF_STORAGE_F32F32: integrate_kernel<KF_STORAGE_F32F32, BATCH><<<grid, 256, 0, st>>>(a, b, chunk); break;
+    case KF_STORAGE_F16U16: integrate_kernel<KF_STORAGE_F16U16, BATCH><<<grid, 256, 0, st>>>(a, b, chunk); break;
+    default: integrate_kernel<KF_STORAGE_RG16I, BATCH><<<grid, 256, 0, st>>>(a, b, chunk); break;
+  }
+  return cudaGetLastError();
 }
 
 IntArgs retarget(IntArgs a, const kf_scratch_target* t) {
@@ -333,10 +521,13 @@ IntArgs retarget(IntArgs a, const kf_scratch_target* t) {
 
 int kf_launch_integrate_shape(kf_session* s, int gated, int zc, const kf_scratch_target* t) {
   const IntArgs a = retarget(make_int_args(s, gated), t);
-  dim3 grid((a.nx + 31) / 32, (a.ny + 7) / 8, (a.nz + zc - 1) / zc);
-  launch_int<false>(s->cfg.storage, zc, grid, s->stream, a, IntBatch{nullptr, nullptr, 0});
-  KF_CUDA_TRY(s, cudaGetLastError());
-  kf_note_launch(s);
+  if (brick_count(a) <= kSmallBricks) {
+    KF_CUDA_TRY(s, launch_int_small(s->cfg.storage, s->stream, a));
+    kf_note_launch(s);
+    return KF_OK;
+  }
+  KF_CUDA_TRY(s, launch_int<false>(s->cfg.storage, s->num_sms, plan_blocks(a), zc, s->stream, a, IntBatch{}));
+  kf_note_launch(s, 2);
   return KF_OK;
 }
 
@@ -351,12 +542,12 @@ int kf_batch_prepare_integrate(kf_batch* b, const kf_scratch_target* over) {
   b->int_prefix = static_cast<const uint32_t*>(kf_batch_table(b, 4 * (size_t)(n + 1), reinterpret_cast<void**>(&hp)));
   if (!b->int_args || !b->int_prefix) return KF_ERR_CAPACITY;
   uint64_t total = 0;
-  const int zc = b->int_zc;
   for (int e = 0; e < n; ++e) {
     // the autotuner's timing runs ungated into scratch copies
     h[e] = over ? retarget(make_int_args(b->members[e], 0), over + e) : make_int_args(b->members[e], 1);
+    h[e].count = b->d_plan + e;
     hp[e] = (uint32_t)total;
-    total += (uint64_t)((h[e].nx + 31) / 32) * ((h[e].ny + 7) / 8) * ((h[e].nz + zc - 1) / zc);
+    total += plan_blocks(h[e]);
   }
   if (total >= (1ull << 31)) return KF_ERR_CAPACITY;
   hp[n] = (uint32_t)total;
@@ -365,9 +556,10 @@ int kf_batch_prepare_integrate(kf_batch* b, const kf_scratch_target* over) {
 }
 
 int kf_batch_launch_integrate(kf_batch* b) {
-  const IntBatch batch = {static_cast<const IntArgs*>(b->int_args), b->int_prefix, (int)b->members.size()};
-  launch_int<true>(b->members[0]->cfg.storage, b->int_zc, dim3(b->int_blocks), b->stream, IntArgs{}, batch);
-  KF_CUDA_TRY(b, cudaGetLastError());
-  b->launches += 1;
+  const IntBatch batch = {static_cast<const IntArgs*>(b->int_args), b->int_prefix, b->d_plan, b->d_plan + b->cap,
+                          (int)b->members.size()};
+  KF_CUDA_TRY(b, launch_int<true>(b->members[0]->cfg.storage, b->num_sms, b->int_blocks, b->int_zc, b->stream, IntArgs{},
+                                  batch));
+  b->launches += 2;
   return KF_OK;
 }

@@ -104,6 +104,9 @@ struct kf_session {
   uint32_t* d_supers = nullptr;
   int sbx = 0, sby = 0, sbz = 0;
   int frames_since_rebuild = 0;  // integrates since the flags were last rebuilt exactly
+  // integrate's plan: the listed bricks' number, the blocks that are through (both zero
+  // between launches), then the list (room for every brick)
+  uint32_t* d_plan = nullptr;
 
   // volume: value plane then weight plane
   void* d_vol = nullptr;
@@ -116,6 +119,9 @@ struct kf_session {
   uint16_t* d_depth_u16 = nullptr;  // upload staging (device)
   float* d_depth_f32_in = nullptr;  // float upload staging (device)
   float* d_depth[3] = {nullptr, nullptr, nullptr};
+  // farthest depth of each 8x8 pixel tile of level 0, then of each 16x16 tile (-inf: no
+  // depth), written with the pyramid and read by integrate's plan
+  float* d_tiles = nullptr;
   float4* d_vertex[3] = {nullptr, nullptr, nullptr};
   float4* d_normal[3] = {nullptr, nullptr, nullptr};
   int32_t* d_status[3] = {nullptr, nullptr, nullptr};
@@ -192,7 +198,7 @@ struct kf_session {
   float4* d_mip = nullptr;  // intensity-projection image, allocated on first use
 
   // launch shapes (kf_set_launch_shape / kf_autotune); every choice computes the same result
-  int int_zc = 16;   // integrate: voxels per thread along z (8, 16, 32)
+  int int_zc = 16;   // integrate: voxels a thread takes per step of the list (8, 16, 32)
   int ray_rows = 4;  // raycast: tile rows of 32 pixels (2, 4, 8), or 1: persistent sweep
 
   // depth ingest before the pyramid (off by default): Kinect-v2 undistortion through a
@@ -240,6 +246,13 @@ struct Vox<KF_STORAGE_F32F32> {
 __device__ __forceinline__ float kf_u16_to_float(uint32_t w) { return __int_as_float(0x4B000000 | w) - 8388608.0f; }
 __device__ __forceinline__ uint32_t kf_float_to_u16_trunc(float w) {
   return (uint32_t)__float_as_int(__fadd_rz(w, 8388608.0f)) & 0xFFFFu;  // 0 <= w <= 65535
+}
+
+// (uint32_t)v * w + (uint32_t)u of 0 <= u, v < 2^23, truncated by adds (the conversion
+// instruction runs at a quarter rate); the two offsets leave in one subtraction
+__device__ __forceinline__ uint32_t kf_trunc_index(float v, float u, uint32_t w) {
+  const uint32_t bv = (uint32_t)__float_as_int(__fadd_rz(v, 8388608.0f)), bu = (uint32_t)__float_as_int(__fadd_rz(u, 8388608.0f));
+  return bv * w + bu - 0x4B000000u * (w + 1u);
 }
 
 template <>
@@ -837,10 +850,11 @@ struct kf_batch {
   int sdf_blocks = 0;
   const void* int_args = nullptr;
   const uint32_t* int_prefix = nullptr;
-  uint32_t int_blocks = 0;
+  uint32_t int_blocks = 0;        // blocks of the batched plan launch
+  unsigned* d_plan = nullptr;     // cap brick counts (one per member) and the done counter
   const void* ray_args = nullptr;
   // launch shapes of the batched integrate and raycast (kf_batch_set_launch_shape /
-  // kf_batch_autotune); the integrate block prefix in the tables depends on int_zc
+  // kf_batch_autotune)
   int int_zc = 16;
   int ray_rows = 4;
   // Steps use two slots in turn, so that an asynchronous step can be enqueued while the
@@ -958,17 +972,24 @@ void kf_scratch_free(kf_scratch_target* t);
 // Tuned shapes remembered per (device, volume size, storage, image size) for new sessions.
 void kf_tune_cache_put(const kf_session* s, int zc, int rows);
 int kf_launch_intensity_projection(kf_session* s, float4* out);
+// Brick flags exact again: kf_refresh_bricks after integrates (only set flags can be stale),
+// kf_rebuild_bricks after the volume was replaced.
+int kf_refresh_bricks(kf_session* s, cudaStream_t stream);
 int kf_rebuild_bricks(kf_session* s, cudaStream_t stream);
 int kf_reset_bricks(kf_session* s);
 int kf_note_integrate(kf_session* s, cudaStream_t stream);
 #define KF_BRICK 8
 #define KF_SUPER 64
+#define KF_PLAN_HEAD 32  // words before the list in kf_session::d_plan
 // Brick flags.  A brick B covers the voxels [8B, 8B+8] on each axis (the taps of every
 // trilinear sample whose base voxel lies in B); a super-brick S covers [64S, 64S+64].
 // NEG: some value there may be negative.  Integrate only ever sets it; an exact rebuild
 // (every KF_BRICK_REBUILD_EVERY integrates, and after a volume upload) clears stale bits,
 // so a clear bit is a guarantee.
+// SET: some value or weight of the brick's own voxels [8B, 8B+8) may have a bit set (a clear
+// bit guarantees a brick of zeros); set and cleared as NEG is.
 #define KF_BRICK_NEG 1u
+#define KF_BRICK_SET 2u
 #define KF_BRICK_REBUILD_EVERY 16
 int kf_mc_run(kf_session* s, float iso, int method, uint32_t* n_tri);
 int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, uint32_t* d_total,

@@ -18,19 +18,29 @@ struct PyrArgs {
   const float* in_f32;
   float* depth[3];
   int W[3], H[3];
+  float* tiles8;   // farthest depth per 8x8 and per 16x16 pixels
+  float* tiles16;
 };
 
-// One thread per level-1 pixel; a 32x8 block also produces a 16x4 level-2 tile.
+__device__ __forceinline__ float far_depth(float d) {
+  if (d == 0.0f) return -INFINITY;
+  return d == d ? fmaxf(d, -3.4e38f) : INFINITY;
+}
+
+// One thread per level-1 pixel; a 32x8 block also produces a 16x4 level-2 tile and, of its
+// 64x16 level-0 pixels, the farthest depth of each 8x8 and 16x16 tile (-inf only where every
+// pixel is 0; a depth that is not a number counts as unbounded).
 // BATCH: blockIdx.z selects the session's arguments in `many`.
 template <bool BATCH>
 __global__ void __launch_bounds__(256) depth_mip_kernel(PyrArgs one, const PyrArgs* many,
                                                         const uint16_t* const* inputs) {
   __shared__ float s_l1[8][33];
+  __shared__ float s_far[8][8];
   PyrArgs a = BATCH ? many[blockIdx.z] : one;
   if (BATCH && inputs) a.in_u16 = inputs[blockIdx.z];  // this step's frame, read in place
   const int x1 = blockIdx.x * 32 + threadIdx.x;
   const int y1 = blockIdx.y * 8 + threadIdx.y;
-  float m = 0.0f;
+  float m = 0.0f, far = -INFINITY;
   if (x1 < a.W[1] && y1 < a.H[1]) {
     const int W0 = a.W[0];
     const size_t i0 = (size_t)(2 * y1) * W0 + 2 * x1;
@@ -46,11 +56,28 @@ __global__ void __launch_bounds__(256) depth_mip_kernel(PyrArgs one, const PyrAr
     }
     *reinterpret_cast<float2*>(a.depth[0] + i0) = make_float2(d00, d01);
     *reinterpret_cast<float2*>(a.depth[0] + i0 + W0) = make_float2(d10, d11);
+    far = fmaxf(fmaxf(far_depth(d00), far_depth(d01)), fmaxf(far_depth(d10), far_depth(d11)));
     m = 0.25f * ((d00 + d01) + (d10 + d11));
     a.depth[1][(size_t)y1 * a.W[1] + x1] = m;
   }
   s_l1[threadIdx.y][threadIdx.x] = m;
+  far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, 1));
+  far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, 2));
+  if ((threadIdx.x & 3) == 0) s_far[threadIdx.y][threadIdx.x >> 2] = far;
   __syncthreads();
+  if (threadIdx.y == 7 && threadIdx.x < 16) {
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const float t8 = fmaxf(fmaxf(s_far[4 * ty][tx], s_far[4 * ty + 1][tx]),
+                           fmaxf(s_far[4 * ty + 2][tx], s_far[4 * ty + 3][tx]));
+    float t16 = fmaxf(t8, __shfl_xor_sync(0xffffu, t8, 1));
+    t16 = fmaxf(t16, __shfl_xor_sync(0xffffu, t16, 8));
+    const int X = blockIdx.x * 8 + tx, Y = blockIdx.y * 2 + ty;
+    const int tw8 = (a.W[0] + 7) / 8, tw16 = (a.W[0] + 15) / 16;
+    if (X < tw8 && Y < (a.H[0] + 7) / 8) {
+      a.tiles8[(size_t)Y * tw8 + X] = t8;
+      if ((tx & 1) == 0 && ty == 0) a.tiles16[(size_t)blockIdx.y * tw16 + (X >> 1)] = t16;
+    }
+  }
   if (threadIdx.x < 16 && threadIdx.y < 4) {
     const int x2 = blockIdx.x * 16 + threadIdx.x;
     const int y2 = blockIdx.y * 4 + threadIdx.y;
@@ -172,6 +199,8 @@ PyrArgs make_pyr_args(kf_session* s, const uint16_t* d_u16, const float* d_f32) 
     a.W[l] = s->W[l];
     a.H[l] = s->H[l];
   }
+  a.tiles8 = s->d_tiles;
+  a.tiles16 = s->d_tiles + (size_t)((s->W[0] + 7) / 8) * ((s->H[0] + 7) / 8);
   return a;
 }
 

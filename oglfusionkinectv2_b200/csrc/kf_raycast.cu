@@ -398,81 +398,112 @@ __global__ void __launch_bounds__(128) mip_kernel(RayArgs a, float4* out) {
   out[(size_t)y * a.W + x] = make_float4(sum, 0.0f, 0.0f, 1.0f);
 }
 
-// Exact NEG flags from the volume itself: a brick B is NEG when a value over the voxels
-// [8B, 8B+8] (clamped to the volume) is negative, a super-brick when one of its 8^3 bricks
-// is (super-bricks are cleared first and set here).  A block takes one row of 32 bricks
-// along x at brick (y, z): thread t scans voxel column x0 + t over the brick's 9 x 9 (y, z)
-// window (coalesced along x), the extra warp the first columns of the next row (the +1
-// layer of the last brick), and thread c merges brick c's 9 columns from shared memory.
-constexpr int kRebuildThreads = 256 + 32;
-
+// Exact brick flags from the volume itself: only a brick whose flag is set can lose it, so a
+// block reads 32 flag words, and its 8 warps check the set ones against the volume, three
+// planes at a time until each set bit is confirmed: NEG by a negative value over the voxels
+// [8B, 8B+8], SET by a nonzero bit in a value or weight of [8B, 8B+8).  Super-bricks are
+// cleared first and set here.  The set bricks come in runs along x, hence few words per block
+// (at most four bricks in a row for a warp, whose latency the launch waits for).
 template <int S>
-__global__ void __launch_bounds__(kRebuildThreads) rebuild_bricks_kernel(const void* vol, int nx, int ny, int nz,
-                                                                          int bx, int by, int bz, uint32_t* bricks,
-                                                                          uint32_t* supers, int sbx, int sby) {
-  __shared__ uint8_t s_neg[kRebuildThreads];
-  const typename Vox<S>::V* f = reinterpret_cast<const typename Vox<S>::V*>(vol);
-  const int x = blockIdx.x * 256 + threadIdx.x;
-  const int y0 = 8 * blockIdx.y, y1 = min(y0 + 8, ny - 1);
-  const int z0 = 8 * blockIdx.z, z1 = min(z0 + 8, nz - 1);
-  bool neg = false;
-  if (x < nx)
-    for (int z = z0; z <= z1 && !neg; ++z) {
-      // the plane's (up to) 9 rows are loaded together; the scan stops after a plane
-      const uint32_t base = (uint32_t)x + (uint32_t)nx * (uint32_t)ny * (uint32_t)z;
+__global__ void __launch_bounds__(256) refresh_bricks_kernel(const void* vol, size_t count, int nx, int ny, int nz,
+                                                             int bx, int by, int bz, uint32_t* bricks,
+                                                             uint32_t* supers, int sbx, int sby) {
+  typedef typename Vox<S>::V V;
+  typedef typename Vox<S>::Wt Wt;
+  const V* f = reinterpret_cast<const V*>(vol);
+  const Wt* wt = reinterpret_cast<const Wt*>(reinterpret_cast<const char*>(vol) + count * sizeof(V));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t n = (uint32_t)bx * by * bz, base = blockIdx.x * 32u;
+  const uint32_t word = base + lane < n ? bricks[base + lane] & (KF_BRICK_NEG | KF_BRICK_SET) : 0u;
+  auto bits = [](const auto& v) {
+    uint32_t b = 0;
+    memcpy(&b, &v, sizeof(v));
+    return b;
+  };
+  __syncthreads();  // every warp has read the words that the warps rewrite below
+  int turn = 0;
+  for (unsigned todo = __ballot_sync(0xffffffffu, word != 0); todo; todo &= todo - 1, ++turn) {
+    if ((turn & 7) != warp) continue;
+    const int k = __ffs(todo) - 1;
+    const uint32_t had = __shfl_sync(0xffffffffu, word, k), b = base + k;
+    const int cx = (int)(b % bx), cy = (int)(b / bx % by), cz = (int)(b / ((uint32_t)bx * by));
+    // the lane's columns of a plane: two of the brick's own 64, one of the +1 layer's 17
+    const int x = 8 * cx + (lane & 7), y = 8 * cy + (lane >> 3);
+    const int ex = lane < 9 ? 8 * cx + 8 : 8 * cx + lane - 9, ey = lane < 9 ? 8 * cy + lane : 8 * cy + 8;
+    const bool in0 = x < nx && y < ny, in1 = x < nx && y + 4 < ny, in2 = lane < 17 && ex < nx && ey < ny;
+    const V zero = Vox<S>::encode_value(0.0f);
+    uint32_t found = 0;
+    for (int d0 = 0; d0 <= 8 && (had & ~found); d0 += 3) {
+      V v[3][3];
+      uint32_t i0[3];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const int y = min(y0 + k, y1);  // rows past the volume repeat the last one
-        neg |= Vox<S>::raw(f, base + (uint32_t)nx * (uint32_t)y) < 0.0f;
+      for (int j = 0; j < 3; ++j) {
+        const bool in = 8 * cz + d0 + j < nz;
+        const uint32_t row = (uint32_t)nx * (uint32_t)ny * (uint32_t)(8 * cz + d0 + j);
+        i0[j] = row + (uint32_t)nx * (uint32_t)y + (uint32_t)x;
+        v[j][0] = in && in0 ? f[i0[j]] : zero;
+        v[j][1] = in && in1 ? f[i0[j] + 4u * (uint32_t)nx] : zero;
+        v[j][2] = in && in2 ? f[row + (uint32_t)nx * (uint32_t)ey + (uint32_t)ex] : zero;
       }
-    }
-  s_neg[threadIdx.x] = neg ? 1 : 0;
-  __syncthreads();
-  const int c = threadIdx.x;
-  const int b = blockIdx.x * 32 + c;
-  if (c < 32 && b < bx) {
-    uint8_t m = 0;
+      bool neg = false, set = false;
 #pragma unroll
-    for (int k = 0; k <= 8; ++k) m |= s_neg[8 * c + k];  // columns past nx - 1 hold 0
-    const uint32_t flag = m ? KF_BRICK_NEG : 0u;
-    bricks[(uint32_t)b + (uint32_t)bx * ((uint32_t)blockIdx.y + (uint32_t)by * (uint32_t)blockIdx.z)] = flag;
-    if (flag) {
-      uint32_t* w = &supers[(uint32_t)(b >> 3) +
-                            (uint32_t)sbx * ((uint32_t)(blockIdx.y >> 3) + (uint32_t)sby * (uint32_t)(blockIdx.z >> 3))];
-      if (!(*(volatile uint32_t*)w & KF_BRICK_NEG)) atomicOr(w, KF_BRICK_NEG);
+      for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) neg |= Vox<S>::raw_nc(&v[j][c], 0) < 0.0f;
+        set |= d0 + j < 8 && (bits(v[j][0]) | bits(v[j][1])) != 0;
+      }
+      if ((had & ~found & KF_BRICK_SET) && !__any_sync(0xffffffffu, set)) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (d0 + j < 8 && 8 * cz + d0 + j < nz)
+            set |= (in0 && bits(wt[i0[j]]) != 0) || (in1 && bits(wt[i0[j] + 4u * (uint32_t)nx]) != 0);
+      }
+      if (__any_sync(0xffffffffu, neg)) found |= KF_BRICK_NEG;
+      if (__any_sync(0xffffffffu, set)) found |= KF_BRICK_SET;
+    }
+    found &= had;
+    if (lane == 0) {
+      bricks[b] = found;
+      if (found & KF_BRICK_NEG) {
+        uint32_t* w = &supers[(uint32_t)(cx >> 3) + (uint32_t)sbx * ((uint32_t)(cy >> 3) + (uint32_t)sby * (uint32_t)(cz >> 3))];
+        if (!(*(volatile uint32_t*)w & KF_BRICK_NEG)) atomicOr(w, KF_BRICK_NEG);
+      }
     }
   }
 }
 
 }  // namespace
 
-int kf_rebuild_bricks(kf_session* s, cudaStream_t stream) {
+int kf_refresh_bricks(kf_session* s, cudaStream_t stream) {
   const uint32_t ns = (uint32_t)s->sbx * s->sby * s->sbz;
   KF_CUDA_TRY(s, cudaMemsetAsync(s->d_supers, 0, ns * sizeof(uint32_t), stream));
-  const dim3 grid((s->bx + 31) / 32, s->by, s->bz);
+  const uint32_t nb = (uint32_t)s->bx * s->by * s->bz;
+  const int grid = (int)((nb + 31) / 32);
+#define KF_REFRESH(S)                                                                                               \
+  refresh_bricks_kernel<S><<<grid, 256, 0, stream>>>(s->d_vol, s->vol_count, s->cfg.nx, s->cfg.ny, s->cfg.nz, s->bx, \
+                                                     s->by, s->bz, s->d_bricks, s->d_supers, s->sbx, s->sby)
   switch (s->cfg.storage) {
-    case KF_STORAGE_F32F32:
-      rebuild_bricks_kernel<KF_STORAGE_F32F32><<<grid, kRebuildThreads, 0, stream>>>(
-          s->d_vol, s->cfg.nx, s->cfg.ny, s->cfg.nz, s->bx, s->by, s->bz, s->d_bricks, s->d_supers, s->sbx, s->sby);
-      break;
-    case KF_STORAGE_F16U16:
-      rebuild_bricks_kernel<KF_STORAGE_F16U16><<<grid, kRebuildThreads, 0, stream>>>(
-          s->d_vol, s->cfg.nx, s->cfg.ny, s->cfg.nz, s->bx, s->by, s->bz, s->d_bricks, s->d_supers, s->sbx, s->sby);
-      break;
-    default:
-      rebuild_bricks_kernel<KF_STORAGE_RG16I><<<grid, kRebuildThreads, 0, stream>>>(
-          s->d_vol, s->cfg.nx, s->cfg.ny, s->cfg.nz, s->bx, s->by, s->bz, s->d_bricks, s->d_supers, s->sbx, s->sby);
-      break;
+    case KF_STORAGE_F32F32: KF_REFRESH(KF_STORAGE_F32F32); break;
+    case KF_STORAGE_F16U16: KF_REFRESH(KF_STORAGE_F16U16); break;
+    default: KF_REFRESH(KF_STORAGE_RG16I); break;
   }
+#undef KF_REFRESH
   KF_CUDA_TRY(s, cudaGetLastError());
   kf_note_launch(s, 1);
   s->frames_since_rebuild = 0;
   return KF_OK;
 }
 
+int kf_rebuild_bricks(kf_session* s, cudaStream_t stream) {
+  // a volume from elsewhere: every flag is set, then checked
+  const size_t nb = (size_t)s->bx * s->by * s->bz;
+  KF_CUDA_TRY(s, cudaMemsetAsync(s->d_bricks, KF_BRICK_NEG | KF_BRICK_SET, nb * 4, stream));
+  return kf_refresh_bricks(s, stream);
+}
+
 int kf_note_integrate(kf_session* s, cudaStream_t stream) {
   if (++s->frames_since_rebuild < KF_BRICK_REBUILD_EVERY) return KF_OK;
-  return kf_rebuild_bricks(s, stream);
+  return kf_refresh_bricks(s, stream);
 }
 
 int kf_reset_bricks(kf_session* s) {

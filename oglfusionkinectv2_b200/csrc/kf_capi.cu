@@ -216,20 +216,21 @@ int alloc_volume(kf_session* s) {
   cudaFree(s->d_vol);
   s->d_vol = nullptr;
   cudaFree(s->d_bricks);
-  s->d_bricks = s->d_supers = nullptr;
+  s->d_bricks = nullptr;
+  s->d_neg = nullptr;
   cudaFree(s->d_plan);
   s->d_plan = nullptr;
   s->bx = (s->cfg.nx + KF_BRICK - 1) / KF_BRICK;
   s->by = (s->cfg.ny + KF_BRICK - 1) / KF_BRICK;
   s->bz = (s->cfg.nz + KF_BRICK - 1) / KF_BRICK;
-  s->sbx = (s->cfg.nx + KF_SUPER - 1) / KF_SUPER;
-  s->sby = (s->cfg.ny + KF_SUPER - 1) / KF_SUPER;
-  s->sbz = (s->cfg.nz + KF_SUPER - 1) / KF_SUPER;
+  s->wx = (s->cfg.nx + KF_WORD - 1) / KF_WORD;
+  s->wy = (s->cfg.ny + KF_WORD - 1) / KF_WORD;
+  s->wz = (s->cfg.nz + KF_WORD - 1) / KF_WORD;
   {
-    const size_t nb = (size_t)s->bx * s->by * s->bz, ns = (size_t)s->sbx * s->sby * s->sbz;
-    int rc = dalloc(s, &s->d_bricks, nb + ns);
+    const size_t nb = (size_t)s->bx * s->by * s->bz;
+    int rc = dalloc(s, &s->d_bricks, kf_flag_words(s->bx, s->by, s->bz));
     if (rc) return rc;
-    s->d_supers = s->d_bricks + nb;
+    s->d_neg = reinterpret_cast<unsigned long long*>(s->d_bricks + kf_brick_words(s->bx, s->by, s->bz));
     if ((rc = kf_reset_bricks(s))) return rc;
     if ((rc = dalloc(s, &s->d_plan, KF_PLAN_HEAD + nb))) return rc;
     KF_CUDA_TRY(s, cudaMemsetAsync(s->d_plan, 0, KF_PLAN_HEAD * 4, s->stream));
@@ -413,7 +414,7 @@ void kf_scratch_free(kf_scratch_target* t) {
 int kf_scratch_alloc(kf_session* s, kf_scratch_target* t) {
   *t = kf_scratch_target{};
   const size_t px = (size_t)s->W[0] * s->H[0];
-  const size_t nflags = (size_t)s->bx * s->by * s->bz + (size_t)s->sbx * s->sby * s->sbz;
+  const size_t nflags = kf_flag_words(s->bx, s->by, s->bz);
   int rc = KF_OK;
   char* vol = nullptr;
   float4* maps = nullptr;
@@ -425,7 +426,7 @@ int kf_scratch_alloc(kf_session* s, kf_scratch_target* t) {
     return rc;
   }
   t->vol = vol;
-  t->supers = t->bricks + (size_t)s->bx * s->by * s->bz;
+  t->neg = reinterpret_cast<unsigned long long*>(t->bricks + kf_brick_words(s->bx, s->by, s->bz));
   t->out_v = maps;
   t->out_n = maps + px;
   KF_CUDA_TRY(s, cudaMemcpyAsync(t->vol, s->d_vol, s->vol_bytes, cudaMemcpyDeviceToDevice, s->stream));
@@ -522,10 +523,9 @@ int kf_session_device_bytes(const kf_config* cfg, const kf_intrinsics* in, uint6
   const uint64_t vox = (uint64_t)cfg->nx * cfg->ny * cfg->nz;
   const uint64_t px = (uint64_t)in->width * in->height;
   uint64_t b = vox * value_bytes(cfg->storage) * 2;
-  b += (uint64_t)((cfg->nx + KF_BRICK - 1) / KF_BRICK) * ((cfg->ny + KF_BRICK - 1) / KF_BRICK) *
-       ((cfg->nz + KF_BRICK - 1) / KF_BRICK) * 8 +
-       (uint64_t)((cfg->nx + KF_SUPER - 1) / KF_SUPER) * ((cfg->ny + KF_SUPER - 1) / KF_SUPER) *
-       ((cfg->nz + KF_SUPER - 1) / KF_SUPER) * 4;  // brick and super-brick flags, integrate's plan
+  const int bx = (cfg->nx + KF_BRICK - 1) / KF_BRICK, by = (cfg->ny + KF_BRICK - 1) / KF_BRICK,
+            bz = (cfg->nz + KF_BRICK - 1) / KF_BRICK;
+  b += (kf_flag_words(bx, by, bz) + (uint64_t)bx * by * bz) * 4;  // brick flags, integrate's plan
   b += KF_PLAN_HEAD * 4 + tile_count(in->width, in->height) * 4;
   b += px * (2 + 4) + px * 2 * kf_session::kRing;  // staging, and the frame graphs' inputs
   b += px * (4 + 16 + 16 + 4) * 2;         // three levels (sum < 4/3 of level 0)

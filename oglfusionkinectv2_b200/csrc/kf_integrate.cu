@@ -35,8 +35,8 @@ struct IntArgs {
   const KfDevState* st;
   uint32_t* bricks;
   int bx, by, bz;
-  uint32_t* supers;
-  int sbx, sby, sbz;
+  unsigned long long* neg;
+  int wx, wy;
   // the farthest depths of 8x8 and 16x16 pixel tiles (kf_pyramid.cu)
   const float* tiles8;
   const float* tiles16;
@@ -347,8 +347,8 @@ __device__ __forceinline__ void integrate_half_brick(const IntArgs& a, uint32_t 
       }
   }
   // Brick flags: lane c merges corner c of the dilation (a brick's low x, y or z layer is
-  // also the +1 layer of the brick below it) and sets the brick's and its super-brick's bit
-  // where it is still clear.
+  // also the +1 layer of the brick below it) and sets the brick's flags where they are still
+  // clear (and with a new NEG its bit).
   const unsigned b_set = __ballot_sync(0xffffffffu, set), b_neg = __ballot_sync(0xffffffffu, neg),
                  b_neg0 = __ballot_sync(0xffffffffu, neg0);
   if (lane < 8 && (b_set | b_neg)) {
@@ -360,11 +360,9 @@ __device__ __forceinline__ void integrate_half_brick(const IntArgs& a, uint32_t 
     if (lane == 0 && b_set) want |= KF_BRICK_SET;
     if (want && gx >= 0 && gy >= 0 && gz >= 0) {
       uint32_t* w = &a.bricks[(uint32_t)gx + (uint32_t)a.bx * ((uint32_t)gy + (uint32_t)a.by * (uint32_t)gz)];
-      if (want & ~*(volatile uint32_t*)w) atomicOr(w, want);
-      if (want & KF_BRICK_NEG) {
-        w = &a.supers[(uint32_t)(gx >> 3) + (uint32_t)a.sbx * ((uint32_t)(gy >> 3) + (uint32_t)a.sby * (uint32_t)(gz >> 3))];
-        if (!(*(volatile uint32_t*)w & KF_BRICK_NEG)) atomicOr(w, KF_BRICK_NEG);
-      }
+      const uint32_t had = *(volatile uint32_t*)w;
+      if (want & ~had) atomicOr(w, want);
+      if (want & ~had & KF_BRICK_NEG) atomicOr(a.neg + kf_neg_word(gx, gy, gz, a.wx, a.wy), kf_neg_bit(gx, gy, gz));
     }
   }
 }
@@ -461,8 +459,8 @@ IntArgs make_int_args(kf_session* s, int gated) {
   a.st = s->d_state;
   a.bricks = s->d_bricks;
   a.bx = s->bx; a.by = s->by; a.bz = s->bz;
-  a.supers = s->d_supers;
-  a.sbx = s->sbx; a.sby = s->sby; a.sbz = s->sbz;
+  a.neg = s->d_neg;
+  a.wx = s->wx; a.wy = s->wy;
   a.tiles8 = s->d_tiles;
   a.tw8 = (a.W + 7) / 8;
   a.tiles16 = s->d_tiles + (size_t)a.tw8 * ((a.H + 7) / 8);
@@ -512,7 +510,7 @@ IntArgs retarget(IntArgs a, const kf_scratch_target* t) {
   if (t) {
     a.vol = t->vol;
     a.bricks = t->bricks;
-    a.supers = t->supers;
+    a.neg = t->neg;
   }
   return a;
 }

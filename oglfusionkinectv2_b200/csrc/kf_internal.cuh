@@ -76,7 +76,7 @@ static_assert(KF_STATE_RESULT_BYTES == 144, "frame result head: pose, tracked, e
 struct kf_scratch_target {
   void* vol;             // integrate: a copy of the volume
   uint32_t* bricks;      // and of the brick / super-brick flags
-  uint32_t* supers;
+  unsigned long long* neg;
   float4* out_v;         // raycast: vertex and normal maps
   float4* out_n;
   KfDevState* st_out;    // raycast: the control block that receives raycast_pose
@@ -99,10 +99,10 @@ struct kf_session {
   // hold a negative TSDF value; set by integrate, cleared by reset, rebuilt on upload
   uint32_t* d_bricks = nullptr;
   int bx = 0, by = 0, bz = 0;
-  // per 64^3 super-brick (8^3 bricks; same allocation as d_bricks, after it): KF_BRICK_NEG
-  // when some brick in it is NEG
-  uint32_t* d_supers = nullptr;
-  int sbx = 0, sby = 0, sbz = 0;
+  // the NEG flags as bits, one word per 4^3 bricks (same allocation as d_bricks, after it):
+  // what the raycast reads
+  unsigned long long* d_neg = nullptr;
+  int wx = 0, wy = 0, wz = 0;
   int frames_since_rebuild = 0;  // integrates since the flags were last rebuilt exactly
   // integrate's plan: the listed bricks' number, the blocks that are through (both zero
   // between launches), then the list (room for every brick)
@@ -979,10 +979,10 @@ int kf_rebuild_bricks(kf_session* s, cudaStream_t stream);
 int kf_reset_bricks(kf_session* s);
 int kf_note_integrate(kf_session* s, cudaStream_t stream);
 #define KF_BRICK 8
-#define KF_SUPER 64
+#define KF_WORD 32  // voxels per side of a NEG word's 4^3 bricks
 #define KF_PLAN_HEAD 32  // words before the list in kf_session::d_plan
 // Brick flags.  A brick B covers the voxels [8B, 8B+8] on each axis (the taps of every
-// trilinear sample whose base voxel lies in B); a super-brick S covers [64S, 64S+64].
+// trilinear sample whose base voxel lies in B).
 // NEG: some value there may be negative.  Integrate only ever sets it; an exact rebuild
 // (every KF_BRICK_REBUILD_EVERY integrates, and after a volume upload) clears stale bits,
 // so a clear bit is a guarantee.
@@ -990,6 +990,18 @@ int kf_note_integrate(kf_session* s, cudaStream_t stream);
 // bit guarantees a brick of zeros); set and cleared as NEG is.
 #define KF_BRICK_NEG 1u
 #define KF_BRICK_SET 2u
+// Where brick (x, y, z) keeps its NEG bit (d_neg): the word, and the bit in it.
+__host__ __device__ inline uint32_t kf_neg_word(int x, int y, int z, int wx, int wy) {
+  return (uint32_t)(x >> 2) + (uint32_t)wx * ((uint32_t)(y >> 2) + (uint32_t)wy * (uint32_t)(z >> 2));
+}
+__host__ __device__ inline unsigned long long kf_neg_bit(int x, int y, int z) {
+  return 1ull << ((x & 3) | (y & 3) << 2 | (z & 3) << 4);
+}
+// 4-byte words of both flag arrays of a volume (the bits start on an 8-byte boundary).
+inline size_t kf_brick_words(int bx, int by, int bz) { return ((size_t)bx * by * bz + 1) & ~(size_t)1; }
+inline size_t kf_flag_words(int bx, int by, int bz) {
+  return kf_brick_words(bx, by, bz) + 2 * (size_t)((bx + 3) / 4) * ((by + 3) / 4) * ((bz + 3) / 4);
+}
 #define KF_BRICK_REBUILD_EVERY 16
 int kf_mc_run(kf_session* s, float iso, int method, uint32_t* n_tri);
 int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, uint32_t* d_total,

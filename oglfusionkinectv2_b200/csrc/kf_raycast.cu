@@ -14,9 +14,15 @@
 // trilinear taps share L1 lines; the value plane alone is read (2 B per tap for the
 // 16-bit storages).  The march position is t0 + k * step (one rounding) rather than the
 // reference's repeated float addition.  Once the march is in its fine-step phase it
-// skips every brick whose negative-value flag is clear (no sample there can be the first
+// skips every brick that holds no negative value (no sample there can be the first
 // negative one), keeping the sample positions tb + k * step and re-evaluating the sample
-// before a hit for the refinement, so the result is the unskipped march's.
+// before a hit for the refinement, so the result is the unskipped march's.  The flags are
+// read as bits, 4^3 bricks to a word: 32 KB for 512^3, which stays in L1, and a zero word
+// skips 32 voxels at once.
+// What bounds it: the chain of a ray's samples (13 coarse, 16 skips and 22 fine ones on average
+// at 512^3) and its tail, a few rays of 200 steps that graze surfaces.  Device us per view,
+// one sample at a time with word flags and exactly verified skips -> now: 512^3 102 -> 60,
+// 768^3 293 -> 168, 128^3 46 -> 32, 16 batched sessions 672 -> 567.
 #include "kf_internal.cuh"
 
 namespace {
@@ -35,10 +41,9 @@ struct RayArgs {
   float4* out_n;
   const KfDevState* st;
   KfDevState* st_out;
-  const uint32_t* bricks;
-  int bx, by, bz;
-  const uint32_t* supers;
-  int sbx, sby, sbz;
+  float inv_step;
+  const unsigned long long* neg;  // NEG bits
+  int wx, wy;
 };
 
 // 32 x ROWS pixel tiles (ROWS one of KF_RAY_ROWS, chosen per session: default 4, or the
@@ -55,17 +60,34 @@ struct Sampler {
   __device__ __forceinline__ float tap(int x, int y, int z) const {
     return Vox<S>::raw(f, (uint32_t)x + (uint32_t)nx * (uint32_t)y + sxy * (uint32_t)z);
   }
-  // interpVol (raycast.cs:69-82) before the final * (1/32766); q in voxel coordinates
-  // (world * volSize / volDim - 0.5).  The 8 taps share one base offset.
-  __device__ __forceinline__ float interp_raw(float qx, float qy, float qz) const {
-    const float bx = floorf(qx), by = floorf(qy), bz = floorf(qz);
-    const float fx = qx - bx, fy = qy - by, fz = qz - bz;
-    const int ix = (int)bx, iy = (int)by, iz = (int)bz;
-    const int lx = min(max(ix, 0), nx - 1), ly = min(max(iy, 0), ny - 1), lz = min(max(iz, 0), nz - 1);
-    const int ux = max(min(ix + 1, nx - 1), 0), uy = max(min(iy + 1, ny - 1), 0), uz = max(min(iz + 1, nz - 1), 0);
+  // The base voxel of a sample and the weights of its far taps.  floor by an add rounded down
+  // (exact below 2^22): the rounding and conversion instructions run at a quarter rate.
+  struct Cell {
+    int x, y, z;
+    float fx, fy, fz;
+  };
+  static __device__ __forceinline__ int floor_of(float q, float* frac) {
+    constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+    const float t = __fadd_rd(q, kMagic);
+    *frac = q - (t - kMagic);
+    return __float_as_int(t) - 0x4B400000;
+  }
+  static __device__ __forceinline__ Cell cell(float qx, float qy, float qz) {
+    Cell c;
+    c.x = floor_of(qx, &c.fx);
+    c.y = floor_of(qy, &c.fy);
+    c.z = floor_of(qz, &c.fz);
+    return c;
+  }
+  // interpVol (raycast.cs:69-82) before the final * (1/32766), taps clamped to the volume.
+  // The 8 taps share one base offset.
+  __device__ __forceinline__ float interp(const Cell& p) const {
+    const int lx = min(max(p.x, 0), nx - 1), ly = min(max(p.y, 0), ny - 1), lz = min(max(p.z, 0), nz - 1);
+    const int ux = max(min(p.x + 1, nx - 1), 0), uy = max(min(p.y + 1, ny - 1), 0), uz = max(min(p.z + 1, nz - 1), 0);
     const uint32_t b = (uint32_t)lx + (uint32_t)nx * (uint32_t)ly + sxy * (uint32_t)lz;
     const uint32_t ox = (uint32_t)(ux - lx), oy = (uint32_t)(uy - ly) * (uint32_t)nx,
                    oz = (uint32_t)(uz - lz) * sxy;
+    const float fx = p.fx, fy = p.fy, fz = p.fz;
     const float c000 = Vox<S>::raw(f, b), c100 = Vox<S>::raw(f, b + ox);
     const float c010 = Vox<S>::raw(f, b + oy), c110 = Vox<S>::raw(f, b + ox + oy);
     const float c001 = Vox<S>::raw(f, b + oz), c101 = Vox<S>::raw(f, b + ox + oz);
@@ -73,139 +95,186 @@ struct Sampler {
     return ((c000 * (1 - fx) + c100 * fx) * (1 - fy) + (c010 * (1 - fx) + c110 * fx) * fy) * (1 - fz) +
            ((c001 * (1 - fx) + c101 * fx) * (1 - fy) + (c011 * (1 - fx) + c111 * fx) * fy) * fz;
   }
+  // q in voxel coordinates (world * volSize / volDim - 0.5)
+  __device__ __forceinline__ float interp_raw(float qx, float qy, float qz) const { return interp(cell(qx, qy, qz)); }
 };
 
-// One pixel of raycast.cs:133-321 for view rows s_view (m_pose * invK): march, refine,
-// gradient normal; writes the pixel's vertex and normal.
-template <int S>
-__device__ __forceinline__ void raycast_pixel(const RayArgs& a, const float* s_view, int x, int y) {
-  Sampler<S> smp;
-  smp.f = reinterpret_cast<const typename Vox<S>::V*>(a.vol);
-  smp.nx = a.nx; smp.ny = a.ny; smp.nz = a.nz;
-  smp.sxy = (uint32_t)a.nx * (uint32_t)a.ny;
+// An integer 0 <= i < 2^23 as float without a conversion instruction.
+__device__ __forceinline__ float float_of(int i) { return __int_as_float(0x4B000000 | i) - 8388608.0f; }
 
+// A pixel's ray (raycast.cs:133-152) for view rows s_view (m_pose * invK): direction, slab
+// clipped to the near and far planes, and the ray in voxel coordinates:
+// q(t) = (o + d t) * volSize / volDim - 0.5 = q0 + t dq.
+struct Ray {
+  float dx, dy, dz;
+  float tnear, tfar;
+  float q0x, q0y, q0z, dqx, dqy, dqz;
+};
+
+__device__ __forceinline__ Ray make_ray(const RayArgs& a, const float* s_view, int x, int y) {
+  Ray r;
   const float ox = s_view[3], oy = s_view[7], oz = s_view[11];
   const float fxp = (float)x, fyp = (float)y;
-  const float dx = fmaf(s_view[0], fxp, fmaf(s_view[1], fyp, s_view[2]));
-  const float dy = fmaf(s_view[4], fxp, fmaf(s_view[5], fyp, s_view[6]));
-  const float dzv = fmaf(s_view[8], fxp, fmaf(s_view[9], fyp, s_view[10]));
-
+  r.dx = fmaf(s_view[0], fxp, fmaf(s_view[1], fyp, s_view[2]));
+  r.dy = fmaf(s_view[4], fxp, fmaf(s_view[5], fyp, s_view[6]));
+  r.dz = fmaf(s_view[8], fxp, fmaf(s_view[9], fyp, s_view[10]));
   // slab test (raycast.cs:141-152)
-  const float ix = 1.0f / dx, iy = 1.0f / dy, iz = 1.0f / dzv;
+  const float ix = 1.0f / r.dx, iy = 1.0f / r.dy, iz = 1.0f / r.dz;
   const float tbx = -1.0f * ix * ox, tby = -1.0f * iy * oy, tbz = -1.0f * iz * oz;
   const float ttx = ix * (a.dimx - ox), tty = iy * (a.dimy - oy), ttz = iz * (a.dimz - oz);
   const float tminx = fminf(ttx, tbx), tminy = fminf(tty, tby), tminz = fminf(ttz, tbz);
   const float tmaxx = fmaxf(ttx, tbx), tmaxy = fmaxf(tty, tby), tmaxz = fmaxf(ttz, tbz);
   const float largest_tmin = fmaxf(fmaxf(tminx, tminy), fmaxf(tminx, tminz));
   const float smallest_tmax = fminf(fminf(tmaxx, tmaxy), fminf(tmaxx, tmaxz));
-  const float tnear = fmaxf(largest_tmin, a.nearp);
-  const float tfar = fminf(smallest_tmax, a.farp);
+  r.tnear = fmaxf(largest_tmin, a.nearp);
+  r.tfar = fminf(smallest_tmax, a.farp);
+  r.q0x = fmaf(ox, a.sx, -0.5f);
+  r.q0y = fmaf(oy, a.sy, -0.5f);
+  r.q0z = fmaf(oz, a.sz, -0.5f);
+  r.dqx = r.dx * a.sx;
+  r.dqy = r.dy * a.sy;
+  r.dqz = r.dz * a.sz;
+  return r;
+}
 
+// Empty-space skipping in the fine phase.  A sample's eight taps lie in the brick of its base
+// voxel; a brick without a negative value (or 4^3 of them, a zero word) cannot hold the first
+// negative sample.  Such samples change nothing but f_t, so the march jumps to the first
+// sample past the region's exit plane; the positions stay tb + k * step, as in the unskipped
+// march.  Exit along an axis: t = edge * r + e with r the reciprocal slope; e moves the plane
+// inwards by more than the positions' rounding, so that every skipped sample lies in the
+// region.
+struct Exits {
+  float rx, ry, rz, ex, ey, ez;
+};
+
+__device__ __forceinline__ Exits make_exits(const RayArgs& a, const Ray& ray) {
+  Exits v;
+  auto axis = [](float dq, float q0, int n, float* r, float* e) {
+    *r = dq != 0.0f ? 1.0f / dq : 0.0f;
+    *e = dq != 0.0f ? -q0 * *r - (0.01f + 1e-6f * (fabsf(q0) + (float)n)) * fabsf(*r) : 1e30f;
+  };
+  axis(ray.dqx, ray.q0x, a.nx, &v.rx, &v.ex);
+  axis(ray.dqy, ray.q0y, a.ny, &v.ry, &v.ey);
+  axis(ray.dqz, ray.q0z, a.nz, &v.rz, &v.ez);
+  return v;
+}
+
+// The NEG words a ray passes, the last one kept.
+struct NegWord {
+  uint32_t at = 0xffffffffu;
+  unsigned long long word = 0;
+};
+
+// Whether the sample in cell p of a fine march (from tb) may be negative; else *next is the
+// number of the first sample past the region without a negative value that p lies in.
+template <class Cell>
+__device__ __forceinline__ bool may_be_negative(const RayArgs& a, const Ray& ray, const Exits& v, const Cell& p,
+                                                float tb, NegWord* nw, float* next) {
+  const int vx = min(max(p.x, 0), a.nx - 1), vy = min(max(p.y, 0), a.ny - 1), vz = min(max(p.z, 0), a.nz - 1);
+  const uint32_t w = kf_neg_word(vx >> 3, vy >> 3, vz >> 3, a.wx, a.wy);
+  if (w != nw->at) {
+    nw->at = w;
+    nw->word = __ldg(a.neg + w);
+  }
+  if (nw->word >> ((vx >> 3 & 3) | (vy >> 3 & 3) << 2 | (vz >> 3 & 3) << 4) & 1u) return true;
+  const int sh = nw->word ? 3 : 5;
+  const float te = fminf(fminf(fmaf(float_of(((vx >> sh) + (ray.dqx > 0.0f)) << sh), v.rx, v.ex),
+                               fmaf(float_of(((vy >> sh) + (ray.dqy > 0.0f)) << sh), v.ry, v.ey)),
+                         fmaf(float_of(((vz >> sh) + (ray.dqz > 0.0f)) << sh), v.rz, v.ez));
+  *next = floorf((fminf(te, ray.tfar) - tb) * a.inv_step) + 1.0f;
+  return false;
+}
+
+// The sample number after k; from 2^24 on the next one that exists (a march of that many steps
+// visits every representable position, as with integer numbers rounded to float).
+__device__ __forceinline__ float after(float k) {
+  const float r = k + 1.0f;
+  return r > k ? r : __int_as_float(__float_as_int(k) + 1);
+}
+
+// Samples a thread takes together.  One 512 x 424 view is 46 warps per SM, too few to hide the
+// taps' latency one sample at a time; a batch fills the GPU and is bound by issue, where
+// discarded samples cost (device us at 1 / 2 / 3 / 4 samples: 512^3 79 / 65 / 60 / 58, 768^3
+// 259 / 190 / 168 / 163, 128^3 37 / 33 / 32 / 33; 16 batched sessions 578 / 567 / 604 / 655).
+constexpr int kAheadOne = 3, kAheadBatch = 2;
+
+// raycast.cs:153-199 for one ray by one thread: the hit's t, 0 for a miss.  AHEAD consecutive
+// samples are taken together and examined in order (the positions do not depend on the
+// samples); those past the first that matters are discarded.
+template <int S, int AHEAD>
+__device__ __forceinline__ float march_ray(const RayArgs& a, const Sampler<S>& smp, const Ray& ray) {
+  if (!(ray.tnear < ray.tfar)) return 0.0f;
   const float scale = Vox<S>::kRawToF;
-  float hx = 0.f, hy = 0.f, hz = 0.f, ht = 0.f;
-  if (tnear < tfar) {
-    float t = tnear, stepsize = a.large_step;
-    // the ray in voxel coordinates: q(t) = (o + d t) * volSize / volDim - 0.5
-    const float q0x = fmaf(ox, a.sx, -0.5f), q0y = fmaf(oy, a.sy, -0.5f), q0z = fmaf(oz, a.sz, -0.5f);
-    const float dqx = dx * a.sx, dqy = dy * a.sy, dqz = dzv * a.sz;
-    auto sample = [&](float tt) {
-      return smp.interp_raw(fmaf(tt, dqx, q0x), fmaf(tt, dqy, q0y), fmaf(tt, dqz, q0z)) * scale;
-    };
-    float f_t = sample(t), f_tt = 0.0f;
-    if (f_t >= 0.0f) {
-      // 1 / ray slope in voxel coordinates, for the brick-exit distances
-      const float rdx = 1.0f / dqx, rdy = 1.0f / dqy, rdz = 1.0f / dqz;
-      float tb = t;
-      int k = 0;
-      bool fine = false;       // stepsize == step (the reference never switches back)
-      bool prev_known = true;  // f_t holds the sample just before t
-      // bounded march: a NaN sample keeps largeStep, so cap the step count
-      for (int n = 0; t < tfar && n < a.max_steps; ++n) {
-        {
-          // empty-space skipping in the fine phase.  A sample's eight taps lie in the brick
-          // (and super-brick) of its base voxel; a region without a negative value cannot
-          // hold the first negative sample.  Such samples change nothing but f_t, so jump to
-          // the first sample past the region; the positions stay tb + k * stepsize, as in
-          // the unskipped march.
-          const float qx = fmaf(t, dqx, q0x), qy = fmaf(t, dqy, q0y), qz = fmaf(t, dqz, q0z);
-          const int vx = min(max((int)floorf(qx), 0), a.nx - 1);
-          const int vy = min(max((int)floorf(qy), 0), a.ny - 1);
-          const int vz = min(max((int)floorf(qz), 0), a.nz - 1);
-          int cell = 0;  // 0: sample it; else the side of the region to skip (64 or 8)
-          int cx = 0, cy = 0, cz = 0, ncx = 1, ncy = 1, ncz = 1;
-          if (fine) {
-            if (!(__ldg(a.supers + (uint32_t)(vx >> 6) +
-                        (uint32_t)a.sbx * ((uint32_t)(vy >> 6) + (uint32_t)a.sby * (uint32_t)(vz >> 6))) &
-                  KF_BRICK_NEG)) {
-              cell = 64;
-              cx = vx >> 6; cy = vy >> 6; cz = vz >> 6;
-              ncx = a.sbx; ncy = a.sby; ncz = a.sbz;
-            } else if (!(__ldg(a.bricks + (uint32_t)(vx >> 3) +
-                               (uint32_t)a.bx * ((uint32_t)(vy >> 3) + (uint32_t)a.by * (uint32_t)(vz >> 3))) &
-                         KF_BRICK_NEG)) {
-              cell = 8;
-              cx = vx >> 3; cy = vy >> 3; cz = vz >> 3;
-              ncx = a.bx; ncy = a.by; ncz = a.bz;
-            }
-          }
-          if (cell) {
-            // the region spans [cell*i, cell*(i+1)) in voxel coordinates; the border ones
-            // extend outwards (taps are clamped there)
-            const float c = (float)cell;
-            float te = tfar;
-            if (dqx > 0.0f && cx < ncx - 1) te = fminf(te, (float)(cx + 1) * c * rdx - q0x * rdx);
-            if (dqx < 0.0f && cx > 0) te = fminf(te, (float)cx * c * rdx - q0x * rdx);
-            if (dqy > 0.0f && cy < ncy - 1) te = fminf(te, (float)(cy + 1) * c * rdy - q0y * rdy);
-            if (dqy < 0.0f && cy > 0) te = fminf(te, (float)cy * c * rdy - q0y * rdy);
-            if (dqz > 0.0f && cz < ncz - 1) te = fminf(te, (float)(cz + 1) * c * rdz - q0z * rdz);
-            if (dqz < 0.0f && cz > 0) te = fminf(te, (float)cz * c * rdz - q0z * rdz);
-            const float kf = ceilf((te - tb) / stepsize);
-            int kn = kf < 2.0e9f ? (int)kf : k + 1;
-            if (kn > k + 1) {
-              // te carries rounding; the rounded sample positions are monotone in k on
-              // every axis, so if the last skipped sample is still in this region, all of
-              // them are.  Otherwise advance by one sample.
-              const float tl = fmaf((float)(kn - 1), stepsize, tb);
-              const int sh = cell == 64 ? 6 : 3;
-              const int jx = min(max((int)floorf(fmaf(tl, dqx, q0x)), 0), a.nx - 1) >> sh;
-              const int jy = min(max((int)floorf(fmaf(tl, dqy, q0y)), 0), a.ny - 1) >> sh;
-              const int jz = min(max((int)floorf(fmaf(tl, dqz, q0z)), 0), a.nz - 1) >> sh;
-              if (jx != cx || jy != cy || jz != cz) kn = k + 1;
-            } else {
-              kn = k + 1;
-            }
-            k = kn;
-            t = fmaf((float)k, stepsize, tb);
-            prev_known = false;
-            continue;
-          }
-        }
-        f_tt = sample(t);
-        if (f_tt < 0.0f) break;
-        if (f_tt < 0.8f && !fine) {
-          fine = true;
-          stepsize = a.step;
-          tb = t;
-          k = 0;
-        }
+  float t = ray.tnear, stepsize = a.large_step;
+  auto cell = [&](float tt) {
+    return Sampler<S>::cell(fmaf(tt, ray.dqx, ray.q0x), fmaf(tt, ray.dqy, ray.q0y), fmaf(tt, ray.dqz, ray.q0z));
+  };
+  float f_t = smp.interp(cell(t)) * scale;
+  if (!(f_t >= 0.0f)) return 0.0f;
+  const Exits v = make_exits(a, ray);
+  float tb = t;
+  float k = 0.0f;          // sample number since tb
+  bool fine = false;       // stepsize == step (the reference never switches back)
+  bool prev_known = true;  // f_t holds the sample just before t
+  NegWord nw;
+  // bounded march: a NaN sample keeps largeStep, so cap the step count
+  for (int n = 0; t < ray.tfar && n < a.max_steps; ++n) {
+    const auto p = cell(t);
+    float next;
+    if (fine && !may_be_negative(a, ray, v, p, tb, &nw, &next)) {
+      k = fmaxf(after(k), next);
+      t = fmaf(k, stepsize, tb);
+      prev_known = false;
+      continue;
+    }
+    float ts[AHEAD], fs[AHEAD];
+    ts[0] = t;
+    fs[0] = smp.interp(p) * scale;
+#pragma unroll
+    for (int i = 1; i < AHEAD; ++i) {
+      ts[i] = fmaf(k + (float)i, stepsize, tb);
+      fs[i] = smp.interp(cell(ts[i])) * scale;
+    }
+    float f_tt = fs[0];
+    bool on = true;  // the samples so far change nothing but f_t
+#pragma unroll
+    for (int i = 1; i < AHEAD; ++i) {
+      on = on && !(f_tt < (fine ? 0.0f : 0.8f)) && ts[i] < ray.tfar;
+      if (on) {
         f_t = f_tt;
         prev_known = true;
-        ++k;
-        t = fmaf((float)k, stepsize, tb);
-      }
-      if (f_tt < 0.0f) {
-        if (!prev_known) f_t = sample(fmaf((float)(k - 1), stepsize, tb));
-        t = t + stepsize * f_tt / (f_t - f_tt);
-        hx = fmaf(dx, t, ox);
-        hy = fmaf(dy, t, oy);
-        hz = fmaf(dzv, t, oz);
-        ht = t;
+        f_tt = fs[i];
+        k += 1.0f;
+        t = ts[i];
       }
     }
+    if (f_tt < 0.0f) {
+      if (!prev_known) f_t = smp.interp(cell(fmaf(k - 1.0f, stepsize, tb))) * scale;
+      return t + stepsize * f_tt / (f_t - f_tt);
+    }
+    if (f_tt < 0.8f && !fine) {
+      fine = true;
+      stepsize = a.step;
+      tb = t;
+      k = 0.0f;
+    }
+    f_t = f_tt;
+    prev_known = true;
+    k = after(k);
+    t = fmaf(k, stepsize, tb);
   }
+  return 0.0f;
+}
 
+// The pixel's vertex and normal for a hit at ht (0: none).
+template <int S>
+__device__ __forceinline__ void write_pixel(const RayArgs& a, const Sampler<S>& smp, const float* s_view, const Ray& ray,
+                                            int x, int y, float ht) {
+  const float scale = Vox<S>::kRawToF;
   const size_t o = (size_t)y * a.W + x;
   if (ht > 0.0f) {
+    const float hx = fmaf(ray.dx, ht, s_view[3]), hy = fmaf(ray.dy, ht, s_view[7]), hz = fmaf(ray.dz, ht, s_view[11]);
     a.out_v[o] = make_float4(hx, hy, hz, 1.0f);
     // getGradient (raycast.cs:229-276)
     const float qx = hx * a.sx - 0.5f, qy = hy * a.sy - 0.5f, qz = hz * a.sz - 0.5f;
@@ -257,6 +326,15 @@ __device__ __forceinline__ void raycast_pixel(const RayArgs& a, const float* s_v
   }
 }
 
+template <int S>
+__device__ __forceinline__ Sampler<S> make_sampler(const RayArgs& a) {
+  Sampler<S> smp;
+  smp.f = reinterpret_cast<const typename Vox<S>::V*>(a.vol);
+  smp.nx = a.nx; smp.ny = a.ny; smp.nz = a.nz;
+  smp.sxy = (uint32_t)a.nx * (uint32_t)a.ny;
+  return smp;
+}
+
 // view = m_pose * invK (gFusion.cpp:1296) from the FP32 pose rows and float invK; thread
 // t < 12 writes element t of the 3x4 rows.
 __device__ __forceinline__ void raycast_view(const RayArgs& a, float* s_view, int t) {
@@ -270,9 +348,19 @@ __device__ __forceinline__ void raycast_view(const RayArgs& a, float* s_view, in
   s_view[r * 4 + c] = v;
 }
 
+// Lane l of warp w in a 32 x ROWS tile.
+template <int ROWS>
+__device__ __forceinline__ int tile_x(int w, int l) {
+  return ROWS == 2 ? w * 16 + (l & 15) : (w & 3) * 8 + (l & 7);
+}
+template <int ROWS>
+__device__ __forceinline__ int tile_y(int w, int l) {
+  return ROWS == 2 ? l >> 4 : (w >> 2) * 4 + (l >> 3);
+}
+
 // BATCH: blockIdx.z selects the session's arguments in `many`.
 template <int S, bool BATCH, int ROWS>
-__global__ void __launch_bounds__(32 * ROWS) raycast_kernel(RayArgs one, const RayArgs* many) {
+__global__ void __launch_bounds__(32 * ROWS, BATCH ? 28 / ROWS : 1) raycast_kernel(RayArgs one, const RayArgs* many) {
   static_assert(ROWS == 2 || ROWS == 4 || ROWS == 8, "raycast tile rows: 2, 4 or 8");
   __shared__ RayArgs s_args;
   __shared__ float s_view[12];  // rows of m_pose * invK: (R K^-1 | t)
@@ -292,23 +380,18 @@ __global__ void __launch_bounds__(32 * ROWS) raycast_kernel(RayArgs one, const R
   // depths, so a warp's taps share cache lines and its lanes finish together (measured
   // ~1 % faster than a 32 x 1 row per warp)
   const int t = threadIdx.y * 32 + threadIdx.x, w = t >> 5, l = t & 31;
-  int x, y;
-  if constexpr (ROWS == 2) {
-    x = blockIdx.x * 32 + w * 16 + (l & 15);
-    y = blockIdx.y * 2 + (l >> 4);
-  } else {
-    x = blockIdx.x * 32 + (w & 3) * 8 + (l & 7);
-    y = blockIdx.y * ROWS + (w >> 2) * 4 + (l >> 3);
-  }
+  const int x = blockIdx.x * 32 + tile_x<ROWS>(w, l), y = blockIdx.y * ROWS + tile_y<ROWS>(w, l);
   if (x >= a.W || y >= a.H) return;
-  raycast_pixel<S>(a, s_view, x, y);
+  const Sampler<S> smp = make_sampler<S>(a);
+  const Ray ray = make_ray(a, s_view, x, y);
+  write_pixel<S>(a, smp, s_view, ray, x, y, march_ray<S, BATCH ? kAheadBatch : kAheadOne>(a, smp, ray));
 }
 
 // The same rays as a persistent sweep: one block per resident slot, and every warp takes
 // the next row segment of 32 pixels from a device counter until the image is done, so no
 // warp waits for another and long rays do not leave SMs idle at the end of the launch.
 // The last warp to find the queue empty resets the counter (and its own completion count)
-// for the next launch.  Every pixel runs raycast_pixel: the maps are the tiled kernel's.
+// for the next launch.  Every pixel runs the same march: the maps are the tiled kernel's.
 template <int S>
 __global__ void __launch_bounds__(256) raycast_sweep_kernel(RayArgs a, unsigned* queue) {
   __shared__ float s_view[12];
@@ -326,7 +409,11 @@ __global__ void __launch_bounds__(256) raycast_sweep_kernel(RayArgs a, unsigned*
     if (seg >= nseg) break;
     const int y = (int)(seg / (unsigned)segs_x);
     const int x = (int)(seg % (unsigned)segs_x) * 32 + lane;
-    if (x < a.W) raycast_pixel<S>(a, s_view, x, y);
+    if (x < a.W) {
+      const Sampler<S> smp = make_sampler<S>(a);
+      const Ray ray = make_ray(a, s_view, x, y);
+      write_pixel<S>(a, smp, s_view, ray, x, y, march_ray<S, kAheadOne>(a, smp, ray));
+    }
   }
   // every warp drew one ticket past the end; the last of them resets the queue
   if (lane == 0) {
@@ -401,13 +488,13 @@ __global__ void __launch_bounds__(128) mip_kernel(RayArgs a, float4* out) {
 // Exact brick flags from the volume itself: only a brick whose flag is set can lose it, so a
 // block reads 32 flag words, and its 8 warps check the set ones against the volume, three
 // planes at a time until each set bit is confirmed: NEG by a negative value over the voxels
-// [8B, 8B+8], SET by a nonzero bit in a value or weight of [8B, 8B+8).  Super-bricks are
+// [8B, 8B+8], SET by a nonzero bit in a value or weight of [8B, 8B+8).  The NEG bits are
 // cleared first and set here.  The set bricks come in runs along x, hence few words per block
 // (at most four bricks in a row for a warp, whose latency the launch waits for).
 template <int S>
 __global__ void __launch_bounds__(256) refresh_bricks_kernel(const void* vol, size_t count, int nx, int ny, int nz,
                                                              int bx, int by, int bz, uint32_t* bricks,
-                                                             uint32_t* supers, int sbx, int sby) {
+                                                             unsigned long long* negs, int wx, int wy) {
   typedef typename Vox<S>::V V;
   typedef typename Vox<S>::Wt Wt;
   const V* f = reinterpret_cast<const V*>(vol);
@@ -464,10 +551,7 @@ __global__ void __launch_bounds__(256) refresh_bricks_kernel(const void* vol, si
     found &= had;
     if (lane == 0) {
       bricks[b] = found;
-      if (found & KF_BRICK_NEG) {
-        uint32_t* w = &supers[(uint32_t)(cx >> 3) + (uint32_t)sbx * ((uint32_t)(cy >> 3) + (uint32_t)sby * (uint32_t)(cz >> 3))];
-        if (!(*(volatile uint32_t*)w & KF_BRICK_NEG)) atomicOr(w, KF_BRICK_NEG);
-      }
+      if (found & KF_BRICK_NEG) atomicOr(negs + kf_neg_word(cx, cy, cz, wx, wy), kf_neg_bit(cx, cy, cz));
     }
   }
 }
@@ -475,13 +559,12 @@ __global__ void __launch_bounds__(256) refresh_bricks_kernel(const void* vol, si
 }  // namespace
 
 int kf_refresh_bricks(kf_session* s, cudaStream_t stream) {
-  const uint32_t ns = (uint32_t)s->sbx * s->sby * s->sbz;
-  KF_CUDA_TRY(s, cudaMemsetAsync(s->d_supers, 0, ns * sizeof(uint32_t), stream));
+  KF_CUDA_TRY(s, cudaMemsetAsync(s->d_neg, 0, (size_t)s->wx * s->wy * s->wz * 8, stream));
   const uint32_t nb = (uint32_t)s->bx * s->by * s->bz;
   const int grid = (int)((nb + 31) / 32);
 #define KF_REFRESH(S)                                                                                               \
   refresh_bricks_kernel<S><<<grid, 256, 0, stream>>>(s->d_vol, s->vol_count, s->cfg.nx, s->cfg.ny, s->cfg.nz, s->bx, \
-                                                     s->by, s->bz, s->d_bricks, s->d_supers, s->sbx, s->sby)
+                                                     s->by, s->bz, s->d_bricks, s->d_neg, s->wx, s->wy)
   switch (s->cfg.storage) {
     case KF_STORAGE_F32F32: KF_REFRESH(KF_STORAGE_F32F32); break;
     case KF_STORAGE_F16U16: KF_REFRESH(KF_STORAGE_F16U16); break;
@@ -508,7 +591,7 @@ int kf_note_integrate(kf_session* s, cudaStream_t stream) {
 
 int kf_reset_bricks(kf_session* s) {
   // an all-zero volume has no negative value
-  const size_t words = (size_t)s->bx * s->by * s->bz + (size_t)s->sbx * s->sby * s->sbz;
+  const size_t words = kf_flag_words(s->bx, s->by, s->bz);
   KF_CUDA_TRY(s, cudaMemsetAsync(s->d_bricks, 0, words * 4, s->stream));
   s->frames_since_rebuild = 0;
   return KF_OK;
@@ -544,10 +627,9 @@ RayArgs make_ray_args(kf_session* s) {
   a.out_n = s->d_ref_normal;
   a.st = s->d_state;
   a.st_out = s->d_state;
-  a.bricks = s->d_bricks;
-  a.bx = s->bx; a.by = s->by; a.bz = s->bz;
-  a.supers = s->d_supers;
-  a.sbx = s->sbx; a.sby = s->sby; a.sbz = s->sbz;
+  a.inv_step = 1.0f / a.step;
+  a.neg = s->d_neg;
+  a.wx = s->wx; a.wy = s->wy;
   return a;
 }
 

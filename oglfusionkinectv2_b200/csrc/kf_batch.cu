@@ -19,14 +19,13 @@
 
 namespace {
 
-// Zero each member's tracking words (barrier counters and ICP sum buffers).
+// Zero each member's tracking words (SDF barrier counter and ICP reduction rows).
 __global__ void batch_clear_kernel(KfDevState* const* states) {
   KfDevState* st = states[blockIdx.x];
   if (threadIdx.x == 0) {
-    st->barrier_count = 0;
     st->sdf_barrier_count = 0;
   }
-  for (int k = threadIdx.x; k < 3 * 32; k += blockDim.x) st->icp_acc[k / 32][k % 32][0] = 0;
+  for (int k = threadIdx.x; k < KF_ICP_WORDS; k += blockDim.x) kf_icp_words(st)[k] = 0;
 }
 
 // Gather each member's frame result (the first KF_STATE_RESULT_BYTES of its state).

@@ -9,11 +9,20 @@
 // (same-pixel projective association at level-0 resolution) and adds the 27 sums of
 // reduce.cs, plus the valid count and the sum of the points, to the session's rows as
 // fixed-point integers (value * 2^32, 64-bit atomics: exact, so the total does not depend
-// on the order or on how the pixels were split among blocks); after a grid barrier every
-// block reads the rows, solves the 6x6 system in FP64 and composes the pose in FP64.  No
+// on the order or on how the pixels were split among blocks); every block waits for the row
+// to be complete, solves the 6x6 system in FP64 and composes the pose in FP64.  No
 // host round trip per iteration (the reference maps the SSBO back every iteration,
 // :1131-1134), no launch per iteration, deterministic sums.  A batched launch gives each
-// session its own group of blocks, rows and barrier.
+// session its own group of blocks and rows.
+//
+// What bounds it: the hand-over between iterations, about 11,000 cycles each (block 0 of a 512^3
+// frame: pixels 3,100, block sums 800, waiting for the row 4,100, solve 1,150, pose 1,800).
+// Device us per frame, before -> now: 128^3 FP32 108 -> 74, 512^3 split-BF16 106-118 -> 81, 16
+// batched sessions 627 -> 544.  What made it: sums that carry their own completeness (no
+// barrier, no second read); two coalesced lines per add (sums interleaved over four lines:
+// 98 us); blocks without pixels add one word; chunks without a valid pixel are left out
+// (batched 600 -> 545); the block's FP32 sums by exchanging halves (88 -> 74).  Slower: two
+// blocks' work in one of 512 threads (93), two or four copies of the row (86, 100).
 
 // Conditioning: J = [n, p x n] with world p couples rotation and translation strongly
 // (lever arms of metres), so FP32 partial sums lose the small eigen-directions of J^T J.
@@ -133,19 +142,55 @@ __device__ __forceinline__ void mma_bf16_16816(float* c, uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Pose (FP64, shared) -> FP32 Ttrack and view = K * inverse(Pv) in shared memory; Pv is
-// the current estimate (Q4, gFusion.cpp:747) or the raycast pose.
-__device__ __forceinline__ void make_float_mats(const IcpArgs& a, const double* P, const double* Pv,
-                                                float* T, float* V) {
-  double inv[16], K[16], view[16];
-  kf_rigid_inverse(a.same_pixel ? P : Pv, inv);
-  for (int i = 0; i < 16; ++i) K[i] = 0;
-  K[0] = a.fx; K[8] = a.cx; K[5] = a.fy; K[9] = a.cy; K[10] = 1; K[15] = 1;
-  kf_mat4_mul(K, inv, view);
-  for (int i = 0; i < 16; ++i) {
-    T[i] = (float)P[i];
-    V[i] = (float)view[i];
+// Element (r, col) of view = K * inverse(Pv) in FP32; Pv is the current estimate (Q4,
+// gFusion.cpp:747) or the raycast pose.
+__device__ __forceinline__ float view_element(const IcpArgs& a, const double* Pv, int r, int col) {
+  // column col of inverse(Pv) = [R^T, -R^T t]
+  double v[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    v[k] = col < 3 ? Pv[k * 4 + col] : -(Pv[k * 4] * Pv[12] + Pv[k * 4 + 1] * Pv[13] + Pv[k * 4 + 2] * Pv[14]);
+  const double w = col < 3 ? 0.0 : 1.0;
+  if (r == 0) return (float)(a.fx * v[0] + a.cx * v[2]);
+  if (r == 1) return (float)(a.fy * v[1] + a.cy * v[2]);
+  return (float)(r == 2 ? v[2] : w);
+}
+
+// One block's share of sum `lane`, added to a reduction row (see kf_icp_words).  A block that
+// has no pixels on this level arrives by the last word alone, which counts every block.
+__device__ __forceinline__ void add_sum(unsigned long long* row, int lane, long long v) {
+  const unsigned long long one = 1ull << 48;
+  atomicAdd(row + lane, one | (uint32_t)v);
+  atomicAdd(row + 32 + lane, one | (uint32_t)((uint32_t)(v >> 32) + 0x80000000u));
+}
+
+__device__ __forceinline__ void arrive(unsigned long long* row) {
+  atomicAdd(row + 63, 1ull << 48 | 0x80000000ull);
+}
+
+// Sum `lane` of a reduction row once all nb blocks have added theirs; the whole warp waits for
+// all 32 sums.  Bounded: after KF_BARRIER_SPIN_CYCLES, or when another block has given up, the
+// error is recorded and false returned.
+__device__ __forceinline__ bool wait_sum(KfDevState* st, const unsigned long long* row, int lane, unsigned nb,
+                                         unsigned active, long long* sum) {
+  const unsigned long long mask = (1ull << 48) - 1ull;
+  unsigned long long lo = 0, hi = 0;
+  const long long t0 = clock64();
+  for (unsigned n = 1;; ++n) {
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(lo) : "l"(row + lane) : "memory");
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(hi) : "l"(row + 32 + lane) : "memory");
+    if (__all_sync(0xffffffffu, (unsigned)(lo >> 48) == active &&
+                                    (unsigned)(hi >> 48) == (lane == 31 ? nb : active)))
+      break;
+    __nanosleep(100);
+    if ((n & 63u) == 0) {
+      const bool late = clock64() - t0 > KF_BARRIER_SPIN_CYCLES;
+      if (late && lane == 0) atomicExch(&st->error, KF_DEV_ERR_TIMEOUT);
+      if (__any_sync(0xffffffffu, late || *(volatile int*)&st->error)) return false;
+    }
   }
+  *sum = (long long)((((hi & mask) - (hi >> 48) * 0x80000000ull) << 32) + (lo & mask));
+  return true;
 }
 
 constexpr int kWarps = KF_TRACK_THREADS / 32;
@@ -156,15 +201,14 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
   __shared__ double s_pose[16];
   __shared__ double s_old[16];
   __shared__ double s_ray[16];
-  __shared__ double s_cd[3];
+  __shared__ double s_centre[2][3];  // this iteration's centre and the next one's, in turn
   __shared__ float s_T[16], s_V[16], s_c[3];
-  __shared__ float s_warp[JTJ ? 1 : kWarps][28];
-  __shared__ float s_pw[JTJ ? 1 : kWarps][4];
+  __shared__ float s_warp[JTJ ? 1 : kWarps][32];
   __shared__ long long s_fix[JTJ ? kWarps : 1][72];
   __shared__ double s_sums[32];
   __shared__ double s_csums[29], s_ccenter[3];  // last centred row (for the tail)
   __shared__ double s_nvalid;                           // its valid-pixel count
-  __shared__ double s_gx[8 + 228];                      // the step (+ rank guard's scratch)
+  __shared__ double s_gx[6 + 228];                      // rank guard: the step, scratch
   __shared__ int s_fast;                                // the rank check's verdict
   __shared__ int s_flag, s_conv;
   __shared__ __align__(16) __nv_bfloat16 s_hi[JTJ ? kWarps : 1][8][40];
@@ -196,20 +240,33 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
     s_ray[tid] = st->raycast_pose[tid];
   }
   __syncthreads();
-  if (tid == 0) {
-    make_float_mats(a, s_pose, s_ray, s_T, s_V);
+  if (tid < 16) {
+    s_T[tid] = (float)s_pose[tid];
+    s_V[tid] = view_element(a, a.same_pixel ? s_pose : s_ray, tid & 3, tid >> 2);
+  }
+  if (tid == 32) {
     // first centre: last frame's centroid, carried in the camera frame
     const double* cc = st->icp_center_cam;
     for (int r = 0; r < 3; ++r) {
-      s_cd[r] = s_pose[r] * cc[0] + s_pose[4 + r] * cc[1] + s_pose[8 + r] * cc[2] + s_pose[12 + r];
-      s_c[r] = (float)s_cd[r];
+      s_centre[0][r] = s_pose[r] * cc[0] + s_pose[4 + r] * cc[1] + s_pose[8 + r] * cc[2] + s_pose[12 + r];
+      s_c[r] = (float)s_centre[0][r];
     }
   }
   __syncthreads();
 
+  // where sum `lane` lies in a warp's 8 x 8 products (row layout of reduce.cs: 0 sum e^2, 1..6
+  // sum J e, 7..27 J^T J (upper, row-major); then 28 valid count, 29..31 sum of the points,
+  // q = hi(p) + mid(p) three words apart)
+  int from;
+  {
+    int r = 0, q = lane - 7;
+    while (q >= 6 - r && r < 5) { q -= 6 - r; ++r; }
+    from = lane == 0 ? 54 : (lane < 7 ? (lane - 1) * 8 + 6 : (lane < 28 ? r * 8 + r + q : (lane == 28 ? 63 : lane + 35)));
+  }
+
   bool ok = true;
   int iters_run = 0;
-  unsigned gi = 0;  // iterations of this launch so far: grid barrier target and sum buffer
+  unsigned gi = 0;  // iterations of this launch so far
   // the first step's vertices and normals of the next iteration, loaded while the current
   // iteration's system is solved (valid when pre_level is the level that runs)
   const float4 none = make_float4(2.0f, 0.f, 0.f, 0.f), zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -225,7 +282,15 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
       c[0] = s_c[0]; c[1] = s_c[1]; c[2] = s_c[2];
 
       // ---------------- track + accumulate ----------------
-      long long* accbuf = &a.st->icp_acc[gi % 3u][0][0];
+      unsigned long long* row = kf_icp_words(st) + (gi % 3u) * KF_ICP_ROW_WORDS;
+      if (local == 0 && warp == 0) {
+        // the next iteration's row, last read two iterations ago; visible before this block's
+        // sums are, and so before any block adds to it
+        unsigned long long* next = kf_icp_words(st) + ((gi + 1u) % 3u) * KF_ICP_ROW_WORDS;
+        next[lane] = 0ull;
+        next[32 + lane] = 0ull;
+        __threadfence();
+      }
       float acc[JTJ ? 1 : 28];
 #pragma unroll
       for (int k = 0; k < (JTJ ? 1 : 28); ++k) acc[k] = 0.0f;
@@ -252,6 +317,7 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
               for (int cc = r; cc < 6; ++cc) acc[q++] += f[r] * f[cc];
           }
         } else {
+          if (!__any_sync(0xffffffffu, use)) return;
           // stage f = [J'0..J'5, e, 1] as hi + mid + lo bf16 and q = [hi(p), mid(p), 0, 0]
           // feature-major per warp (zero for pixels that are not used)
 #pragma unroll
@@ -307,6 +373,7 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
       // passes), so two pixels' gathers are in flight per thread, and the step after that
       // one's vertices and normals are loaded meanwhile.
       const int stride = nb * KF_TRACK_THREADS;
+      const unsigned active = min(nb, (unsigned)(P + KF_TRACK_THREADS - 1) / KF_TRACK_THREADS);  // blocks with pixels
       const float4* Nl = a.normal[level];
       const float4* Vl = a.vertex[level];
       const int first = (local * kWarps + warp) * 32;
@@ -348,26 +415,27 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
 
       // ---------------- block sums -> the entry's fixed-point rows ----------------
       if constexpr (JTJ == 0) {
+        // the 32 sums over the warp by exchanging halves: lane k ends with sum k, added in the
+        // order of a butterfly per sum (31 shuffles instead of 160)
+        float v32[32];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float v = pacc[k];
+        for (int k = 0; k < 32; ++k) v32[k] = k < 28 ? acc[k] : pacc[k - 28];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) s_pw[warp][k] = v;
-        }
+        for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int k = 0; k < 28; ++k) {
-          float v = acc[k];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) s_warp[warp][k] = v;
-        }
+          for (int k = 0; k < o; ++k) {
+            const bool up = lane & o;
+            const float keep = up ? v32[k + o] : v32[k], send = up ? v32[k] : v32[k + o];
+            v32[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        s_warp[warp][lane] = v32[0];
         __syncthreads();
         if (tid < 32) {
           float v = 0.0f;
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w) v += tid < 28 ? s_warp[w][tid] : s_pw[w][tid - 28];
-          atomicAdd(reinterpret_cast<unsigned long long*>(accbuf + tid), (unsigned long long)__float2ll_rn(v * kFix));
+          for (int w = 0; w < kWarps; ++w) v += s_warp[w][lane];
+          if (local < active) add_sum(row, lane, __float2ll_rn(v * kFix));
+          else if (lane == 31) arrive(row);
         }
       } else {
         // lane (g, t) holds M[g][2t], M[g][2t+1]; lanes t == 3 also sum q_g
@@ -377,40 +445,21 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
         if (t == 3) s_fix[warp][64 + g] = fxq;
         __syncthreads();
         if (tid < 32) {
-          // row layout of reduce.cs: 0 sum e^2, 1..6 sum J e, 7..27 J^T J (upper, row-major);
-          // then 28 valid count, 29..31 sum of the points (q = hi(p) + mid(p))
           long long v = 0;
-          if (tid < 28) {
-            int r, cc;
-            if (tid == 0) { r = 6; cc = 6; }
-            else if (tid < 7) { r = tid - 1; cc = 6; }
-            else {
-              int q = tid - 7;
-              r = 0;
-              while (q >= 6 - r) { q -= 6 - r; ++r; }
-              cc = r + q;
-            }
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) v += s_fix[w][r * 8 + cc];
-          } else if (tid == 28) {
+          for (int w = 0; w < kWarps; ++w) v += s_fix[w][from];
+          if (tid > 28) {
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) v += s_fix[w][63];
-          } else {
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) v += s_fix[w][64 + tid - 29] + s_fix[w][64 + tid - 26];
+            for (int w = 0; w < kWarps; ++w) v += s_fix[w][from + 3];
           }
-          atomicAdd(reinterpret_cast<unsigned long long*>(accbuf + tid), (unsigned long long)v);
+          if (local < active) add_sum(row, lane, v);
+          else if (lane == 31) arrive(row);
         }
       }
-      // the buffer of the next iteration was last read before the previous barrier
-      if (local == 0 && tid >= 32 && tid < 64) a.st->icp_acc[(gi + 1u) % 3u][tid - 32][0] = 0;
-
-      // ---------------- grid barrier; then every block solves ----------------
+      // ---------------- every block's sums; then every block solves ----------------
       // Every block reads the same exact sums and solves the same system in FP64, so all
       // blocks hold bit-identical results without a second hand-over, and the solve's code
       // stays warm in every SM's instruction cache.
-      ok = kf_grid_sync(st, &st->barrier_count, nb * (gi + 1u), &s_flag);
-      if (!ok) break;
       {
         // the next iteration runs this level again unless the level's iterations are used up
         // or this solve converges; the first case is known now, the second is rare
@@ -427,56 +476,65 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
           }
         }
       }
-      if (tid < 32) s_sums[tid] = (double)__ldcg(accbuf + tid) * kInvFix;
-      __syncthreads();
+      const double* cd = s_centre[gi & 1u];
+      if (warp < 3) {
+        if (warp == 0) {
+          long long sum = 0;
+          const bool got = wait_sum(st, row, lane, nb, active, &sum);
+          s_sums[lane] = (double)sum * kInvFix;
+          if (lane == 0) s_flag = got ? 1 : 0;
+        }
+        asm volatile("bar.sync 1, 96;" ::: "memory");  // warps 0..2: the sums
+      }
       if (warp == 1) {
         // the rank guard's check (KF_ICP_RANK_TAU), in FP32 by lane 0 beside warp 0's FP64
         // solve (measured 1-2 us per frame faster than the check spread over the warp's lanes)
-        if (lane == 0) s_fast = kf_icp_rank_check_thread(&s_sums[7], s_cd);
-        asm volatile("bar.sync 1, 64;" ::: "memory");  // warps 0 and 1
+        if (lane == 0) s_fast = kf_icp_rank_check_thread(&s_sums[7], cd);
+        asm volatile("bar.sync 2, 64;" ::: "memory");  // warps 0 and 1
+      }
+      if (warp == 2) {
+        // the next centre (this iteration's centroid of the valid points), and what the tail
+        // needs of the last iteration: the centred row, its centre and its counts.
+        // reduce.cs counts every pixel of the (group-7) rows in sums[28]
+        const double nvalid = s_sums[28];
+        if (lane < 28) s_csums[lane] = s_sums[lane];
+        if (lane == 28) s_csums[28] = a.q1 ? (double)Wl * (double)(Hl / 8) : (double)P;
+        if (lane == 31) s_nvalid = nvalid;
+        const int ci = lane < 3 ? lane : 2;
+        const double centroid = s_sums[29 + ci] / nvalid;  // unused when nvalid == 0
+        const double cn = nvalid > 0 ? centroid : cd[ci];
+        if (lane < 3) {
+          s_ccenter[lane] = cd[lane];
+          s_centre[(gi + 1u) & 1u][lane] = cn;
+          s_c[lane] = (float)cn;
+        }
       }
       if (warp == 0) {
-        // ---- solve in warp 0 ----
-        // reduce.cs counts every pixel of the (group-7) rows in sums[28]
-        const double count = a.q1 ? (double)Wl * (double)(Hl / 8) : (double)P;
-        const double nvalid = s_sums[28];
-        const double cx = s_cd[0], cy = s_cd[1], cz = s_cd[2];
-        // lane 0 factors and solves; the step reaches the other lanes through shared memory
+        // ---- solve in warp 0: every lane the same, so nothing has to be handed on ----
         double xp[6];
-        bool spd = false;
-        if (lane == 0) {
-          spd = kf_cholesky6_thread(&s_sums[7], &s_sums[1], xp);
-#pragma unroll
-          for (int k = 0; k < 6; ++k) s_gx[k] = xp[k];
-          s_gx[6] = spd ? 1.0 : 0.0;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < 6; ++k) xp[k] = s_gx[k];
-        spd = s_gx[6] != 0.0;
+        kf_solve6(&s_sums[7], &s_sums[1], xp);
         // back to the reference's variables: w = w', t = t' - w x c
+        const double cx = cd[0], cy = cd[1], cz = cd[2];
         double x[6];
         x[3] = xp[3]; x[4] = xp[4]; x[5] = xp[5];
         x[0] = xp[0] - (x[4] * cz - x[5] * cy);
         x[1] = xp[1] - (x[5] * cx - x[3] * cz);
         x[2] = xp[2] - (x[3] * cy - x[4] * cx);
-        asm volatile("bar.sync 1, 64;" ::: "memory");  // warp 1's rank check is in s_fast
-        if (!(spd && s_fast)) {
+        asm volatile("bar.sync 2, 64;" ::: "memory");  // warp 1's rank check is in s_fast
+        if (!s_fast) {
           // a degenerate view (rare): the rank-guarded minimum-norm step of the world-frame
           // system (JacobiSVD::solve, :696-697, with the cut of KF_ICP_RANK_TAU)
-          if (lane == 0) kf_icp_world_guarded_step(&s_sums[7], &s_sums[1], s_cd, s_gx, s_gx + 8);
+          if (lane == 0) kf_icp_world_guarded_step(&s_sums[7], &s_sums[1], cd, s_gx, s_gx + 6);
           __syncwarp();
 #pragma unroll
           for (int k = 0; k < 6; ++k) x[k] = s_gx[k];
           __syncwarp();
         }
-        // delta = eulerAngleXYZ(x3, x4, x5), delta[3].xyz = x0..2 (gFusion.cpp:700-703);
-        // lanes 0..2 evaluate the three sincos at once
-        double sn, cs;
-        kf_sincos_step(lane == 0 ? x[3] : (lane == 1 ? x[4] : x[5]), &sn, &cs);
-        const double sa = __shfl_sync(0xffffffffu, sn, 0), ca = __shfl_sync(0xffffffffu, cs, 0);
-        const double sb = __shfl_sync(0xffffffffu, sn, 1), cb = __shfl_sync(0xffffffffu, cs, 1);
-        const double sc = __shfl_sync(0xffffffffu, sn, 2), cc = __shfl_sync(0xffffffffu, cs, 2);
+        // delta = eulerAngleXYZ(x3, x4, x5), delta[3].xyz = x0..2 (gFusion.cpp:700-703)
+        double sa, ca, sb, cb, sc, cc;
+        kf_sincos_step(x[3], &sa, &ca);
+        kf_sincos_step(x[4], &sb, &cb);
+        kf_sincos_step(x[5], &sc, &cc);
         double R[9];
         kf_euler_xyz_from_sincos(sa, ca, sb, cb, sc, cc, R);
         // pose = delta * pose, one element per lane (delta column-major: R | x0..2)
@@ -493,34 +551,21 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
           pn += d2 * s_pose[col * 4 + 2];
           pn += d3 * s_pose[col * 4 + 3];
         }
-        // the centred row and its centre; the tail turns the last one into the world form
-        if (lane < 28) s_csums[lane] = s_sums[lane];
-        if (lane == 28) s_csums[28] = count;
-        // the convergence test and the next centre (this iteration's centroid of the valid
-        // points) in every lane: one instruction stream, no divergent FP64 square root or
-        // division on the hand-over's path
-        const double nrm = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3] +
-                                x[4] * x[4] + x[5] * x[5]);
-        if (lane == 29) s_conv = (nrm < 1e-5 && nrm != 0.0) ? 1 : 0;
-        if (lane == 31) s_nvalid = nvalid;
-        const int ci = lane < 3 ? lane : 2;
-        const double centroid = s_sums[29 + ci] / nvalid;  // unused when nvalid == 0
-        const double cn = nvalid > 0 ? centroid : s_cd[ci];
+        // result.norm() < 1e-5 && != 0 (:707), squared
+        const double n2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3] + x[4] * x[4] + x[5] * x[5];
+        if (lane == 29) s_conv = (n2 < 1e-10 && n2 != 0.0) ? 1 : 0;
         __syncwarp();
         if (lane < 16) {
           s_pose[lane] = pn;
           s_T[lane] = (float)pn;
         }
-        if (lane < 3) {
-          s_ccenter[lane] = s_cd[lane];
-          s_cd[lane] = cn;
-          s_c[lane] = (float)cn;
-        }
         __syncwarp();
-        if (a.same_pixel && lane == 0) make_float_mats(a, s_pose, s_ray, s_T, s_V);
+        if (a.same_pixel && lane < 16) s_V[lane] = view_element(a, s_pose, lane & 3, lane >> 2);
       }
-      ++gi;
       __syncthreads();
+      ok = s_flag != 0;
+      if (!ok) break;
+      ++gi;
       ++iters_run;
       if (s_conv) break;  // result.norm() < 1e-5 && != 0 leaves this level (:707-708)
     }
@@ -587,9 +632,10 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
     }
     // keep the centroid for the next frame, in the camera frame of the tracked pose
     double inv[16];
+    const double* cd = s_centre[gi & 1u];
     kf_rigid_inverse(s_pose, inv);
     for (int r = 0; r < 3; ++r)
-      st->icp_center_cam[r] = inv[r] * s_cd[0] + inv[4 + r] * s_cd[1] + inv[8 + r] * s_cd[2] + inv[12 + r];
+      st->icp_center_cam[r] = inv[r] * cd[0] + inv[4 + r] * cd[1] + inv[8 + r] * cd[2] + inv[12 + r];
   }
   for (int k = 0; k < 16; ++k) st->old_pose[k] = s_old[k];
   st->tracked = tracked;

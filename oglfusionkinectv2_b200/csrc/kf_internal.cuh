@@ -19,11 +19,6 @@
 #define KF_BATCH_ICP_WAVE 32     // members per cooperative launch of the batched ICP
 #define KF_MAX_TRACK_BLOCKS 1024  // upper bound of the persistent grid
 
-// Words of 8 bytes between two ICP reduction sums: 1, so that a warp's atomics on the 32
-// sums of a row fall on two 128-byte lines and coalesce (one sum per line measured slower:
-// 32 separate L2 requests per block instead of two).
-#define KF_ACC_STRIDE 1
-
 // Device-side error word values (KfDevState::error).
 #define KF_DEV_ERR_TIMEOUT 1
 
@@ -54,20 +49,29 @@ struct KfDevState {
   int do_integrate;     // frame policy: integrate this frame
   int reset_window;     // kinect.cpp `reset` flag
   int iterations_run;   // ICP/SDF iterations executed by the last tracking call
-  // grid barrier counters, each on its own 128-byte line (polled by every block while the
-  // reduction atomics land elsewhere)
-  alignas(128) unsigned barrier_count;      // grid barrier of the ICP launch
-  alignas(128) unsigned sdf_barrier_count;  // grid barrier of the SDF launch
-  // ICP reduction rows as fixed-point sums (value * 2^32, exact and order-independent),
-  // three buffers used in turn by successive iterations of a launch (KF_ACC_STRIDE words
-  // between sums)
-  alignas(128) long long icp_acc[3][32][KF_ACC_STRIDE];
+  // words no kernel uses any more, kept so that the control block of a saved file keeps its
+  // layout
+  alignas(128) unsigned reserved_count;
+  // grid barrier of the SDF launch, on its own 128-byte line (polled by every block)
+  alignas(128) unsigned sdf_barrier_count;
+  alignas(128) long long reserved_sums[3][32];
   // the persistent raycast sweep's row-segment queue: next segment, warps done (both zero
   // between launches: the sweep's last warp resets them)
   alignas(128) unsigned ray_queue[2];
   double icp_center_cam[3];  // ICP centre at the end of the last frame (camera frame)
   double lib_pose[KF_MAX_LIBRARY][16];  // pose library
 };
+// The ICP launch's reduction rows, in the words after the control block: three rows used in
+// turn by successive iterations, 32 sums each of two words.  A sum is a fixed-point number
+// (value * 2^32, exact and order-independent); its low 32 bits and its high 32 bits (biased by
+// 2^31) are added up in a word each, bits 0..47, beside a count of the blocks that have added
+// theirs in bits 48..63, so that a reader sees a sum and its completeness in one load and the
+// launch needs no other grid barrier.
+#define KF_ICP_ROW_WORDS 64
+#define KF_ICP_WORDS (3 * KF_ICP_ROW_WORDS)
+__host__ __device__ inline unsigned long long* kf_icp_words(KfDevState* st) {
+  return reinterpret_cast<unsigned long long*>(st + 1);
+}
 // Bytes of KfDevState the host reads after a frame step (pose and result flags).
 #define KF_STATE_RESULT_BYTES (offsetof(KfDevState, pose_rows))
 static_assert(KF_STATE_RESULT_BYTES == 144, "frame result head: pose, tracked, error, recover_found, counter");
@@ -385,44 +389,6 @@ __host__ __device__ inline void kf_store_pose(KfDevState* st, const double* P) {
     }
 }
 
-// FP64 Cholesky solve of the 6x6 SPD normal equations.  Returns 0 and x = 0 when a pivot
-// is not positive (rank-deficient C, where the reference's JacobiSVD would return the
-// minimum-norm solution; an all-zero system gives x = 0 in both).
-__host__ __device__ inline int kf_cholesky6(const double* C, const double* b, double* x) {
-  double L[36];
-  for (int i = 0; i < 36; ++i) L[i] = 0;
-  double dmax = 0;
-  for (int i = 0; i < 6; ++i) dmax = fmax(dmax, fabs(C[i * 7]));
-  const double eps = 1e-13 * dmax;
-  for (int j = 0; j < 6; ++j) {
-    double d = C[j * 7];
-    for (int k = 0; k < j; ++k) d -= L[j * 6 + k] * L[j * 6 + k];
-    if (!(d > eps)) {
-      for (int i = 0; i < 6; ++i) x[i] = 0;
-      return 0;
-    }
-    double ljj = sqrt(d);
-    L[j * 7] = ljj;
-    for (int i = j + 1; i < 6; ++i) {
-      double v = C[i * 6 + j];
-      for (int k = 0; k < j; ++k) v -= L[i * 6 + k] * L[j * 6 + k];
-      L[i * 6 + j] = v / ljj;
-    }
-  }
-  double y[6];
-  for (int i = 0; i < 6; ++i) {
-    double v = b[i];
-    for (int k = 0; k < i; ++k) v -= L[i * 6 + k] * y[k];
-    y[i] = v / L[i * 7];
-  }
-  for (int i = 5; i >= 0; --i) {
-    double v = y[i];
-    for (int k = i + 1; k < 6; ++k) v -= L[k * 6 + i] * x[k];
-    x[i] = v / L[i * 7];
-  }
-  return 1;
-}
-
 // LDL^T solve (C.ldlt().solve(b), gFusion.cpp:902), unpivoted; NaN in, NaN out.
 __host__ __device__ inline void kf_ldlt6(const double* C, const double* b, double* x) {
   double L[36], D[6];
@@ -463,15 +429,14 @@ __host__ __device__ inline void kf_make_jtj(const double* v21, double* C) {
     }
 }
 
-// 1 / sqrt(d) to FP64 precision without a divide or square root: an FP32 estimate refined
-// by two Newton-Raphson steps for f(y) = 1/y^2 - d, y <- y (3 - d y^2) / 2; each step
-// roughly doubles the correct bits (22 -> 44 -> FP64 rounding).  Outside FP32's normal
-// range the estimate comes from 1 / sqrt(d) directly.
-__device__ __forceinline__ double kf_rsqrt_newton(double d) {
-  double y = (d > 1e-30 && d < 1e30) ? (double)rsqrtf((float)d) : 1.0 / sqrt(d);
-  const double h = 0.5 * d;
-  y = y * fma(-h * y, y, 1.5);
-  y = y * fma(-h * y, y, 1.5);
+// 1 / d to FP64 precision without a divide: an FP32 estimate refined by two Newton-Raphson
+// steps y <- y + y (1 - d y), each of which doubles the correct bits (23 -> 46 -> FP64
+// rounding).  Outside FP32's normal range the estimate is the quotient itself.
+__device__ __forceinline__ double kf_rcp_newton(double d) {
+  const double m = fabs(d);
+  double y = (m > 1e-30 && m < 1e30) ? (double)__frcp_rn((float)d) : 1.0 / d;
+  y = fma(fma(-d, y, 1.0), y, y);
+  y = fma(fma(-d, y, 1.0), y, y);
   return y;
 }
 
@@ -498,58 +463,50 @@ __device__ __forceinline__ void kf_sincos_step(double x, double* s, double* c) {
   }
 }
 
-// kf_cholesky6 by one thread: C given as the 21 upper-triangular values of reduce.cs rows
-// 7..27 (row-major), b as 6 values, both read from shared or global memory.  Returns
-// whether C was numerically positive definite (x = 0 otherwise, as kf_cholesky6).  Fully
-// unrolled in registers: the dependent chain is six pivots (kf_rsqrt_newton: multiplies,
-// no divides) and twelve substitution steps, with no shuffles between lanes (measured
-// 11 us per frame faster than a lane-per-row warp factorisation, whose every pivot and
-// substitution step waited on a shuffle).
-__device__ __forceinline__ bool kf_cholesky6_thread(const double* v21, const double* b, double* x) {
-  double L[6][6];  // lower triangle
-  double inv[6];
-  double dmax = 0.0;
+// The inverse of a symmetric 3x3 matrix {m00, m01, m02, m11, m12, m22} by its cofactors.
+__device__ __forceinline__ void kf_inverse3(const double* m, double* r) {
+  const double c00 = fma(m[3], m[5], -m[4] * m[4]), c01 = fma(m[2], m[4], -m[1] * m[5]), c02 = fma(m[1], m[4], -m[2] * m[3]);
+  const double c11 = fma(m[0], m[5], -m[2] * m[2]), c12 = fma(m[1], m[2], -m[0] * m[4]), c22 = fma(m[0], m[3], -m[1] * m[1]);
+  const double i = kf_rcp_newton(fma(m[0], c00, fma(m[1], c01, m[2] * c02)));
+  r[0] = c00 * i; r[1] = c01 * i; r[2] = c02 * i;
+  r[3] = c11 * i; r[4] = c12 * i; r[5] = c22 * i;
+}
+__device__ __forceinline__ double kf_row3(const double* m, int i, double x, double y, double z) {
+  // row i of the symmetric matrix times (x, y, z)
+  return i == 0 ? fma(m[0], x, fma(m[1], y, m[2] * z))
+                : (i == 1 ? fma(m[1], x, fma(m[3], y, m[4] * z)) : fma(m[2], x, fma(m[4], y, m[5] * z)));
+}
+
+// The 6x6 normal equations in FP64 by 3x3 blocks: C = [[A, B], [B^T, D]] (v21: the 21
+// upper-triangular values of reduce.cs rows 7..27), the Schur complement S = D - B^T A^-1 B.
+// For a C that passed the rank check.  The dependent chain is two reciprocals and some thirty
+// multiply-adds; a Cholesky factorisation's six pivots and twelve substitution steps were
+// three times as long (and its error against extended precision slightly larger: 1.7e-16
+// against 1.3e-16 median relative over systems of condition 2 to 3e4).
+__device__ __forceinline__ void kf_solve6(const double* v21, const double* b, double* x) {
+  const double A[6] = {v21[0], v21[1], v21[2], v21[6], v21[7], v21[11]};
+  const double B[3][3] = {{v21[3], v21[4], v21[5]}, {v21[8], v21[9], v21[10]}, {v21[12], v21[13], v21[14]}};
+  const double D[6] = {v21[15], v21[16], v21[17], v21[18], v21[19], v21[20]};
+  double Ai[6], W[3][3], S[6], Si[6], y[3], r[3];
+  kf_inverse3(A, Ai);
 #pragma unroll
-  for (int i = 0; i < 6; ++i) dmax = fmax(dmax, fabs(v21[6 * i - (i * (i - 1)) / 2]));
-  const double eps = 1e-13 * dmax;
-  bool spd = true;
+  for (int i = 0; i < 3; ++i) {
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    double dj = v21[6 * j - (j * (j - 1)) / 2];
-#pragma unroll
-    for (int k = 0; k < j; ++k) dj = fma(-L[j][k], L[j][k], dj);
-    spd = spd && (dj > eps);
-    const double r = kf_rsqrt_newton(spd ? dj : 1.0);
-    inv[j] = r;
-    L[j][j] = dj * r;
-#pragma unroll
-    for (int i = j + 1; i < 6; ++i) {
-      double v = v21[6 * j - (j * (j - 1)) / 2 + (i - j)];
-#pragma unroll
-      for (int k = 0; k < j; ++k) v = fma(-L[i][k], L[j][k], v);
-      L[i][j] = v * r;
-    }
+    for (int j = 0; j < 3; ++j) W[i][j] = kf_row3(Ai, i, B[0][j], B[1][j], B[2][j]);  // A^-1 B
+    y[i] = kf_row3(Ai, i, b[0], b[1], b[2]);
   }
-  double y[6];
+  int q = 0;
 #pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double v = b[i];
+  for (int i = 0; i < 3; ++i) {
 #pragma unroll
-    for (int k = 0; k < i; ++k) v = fma(-L[i][k], y[k], v);
-    y[i] = v * inv[i];
+    for (int j = i; j < 3; ++j, ++q) S[q] = fma(-B[0][i], W[0][j], fma(-B[1][i], W[1][j], fma(-B[2][i], W[2][j], D[q])));
+    r[i] = fma(-B[0][i], y[0], fma(-B[1][i], y[1], fma(-B[2][i], y[2], b[3 + i])));
   }
+  kf_inverse3(S, Si);
 #pragma unroll
-  for (int i = 5; i >= 0; --i) {
-    double v = y[i];
+  for (int i = 0; i < 3; ++i) x[3 + i] = kf_row3(Si, i, r[0], r[1], r[2]);
 #pragma unroll
-    for (int k = i + 1; k < 6; ++k) v = fma(-L[k][i], x[k], v);
-    x[i] = spd ? v * inv[i] : 0.0;
-  }
-  if (!spd) {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) x[i] = 0.0;
-  }
-  return spd;
+  for (int i = 0; i < 3; ++i) x[i] = fma(-W[i][0], x[3], fma(-W[i][1], x[4], fma(-W[i][2], x[5], y[i])));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -694,7 +651,7 @@ __device__ inline void kf_icp_world_guarded_step(const double* v21c, const doubl
 
 // The rank guard's check by one thread, in FP32 (run in warp 1 beside warp 0's FP64
 // solve): 1 when the world-frame C provably keeps every direction under
-// KF_ICP_RANK_TAU, so that the centred system's Cholesky solution is the guarded step.
+// KF_ICP_RANK_TAU, so that the centred system's own solution is the guarded step.
 // v21c: reduce.cs rows 7..27 of the centred J' = [n, (p - c) x n] about c, i.e.
 // C' = M^-T C M^-1 with M: t' = t - [c]x w.  Bounds: l_min >= 1 / trace(C^-1),
 // l_max <= trace(C), with trace(C) = sum_i m_i^T C' m_i (m_i = M e_i) and
@@ -929,11 +886,9 @@ int kf_batch_launch_sdf_recover(kf_batch* b);
 int kf_batch_launch_integrate(kf_batch* b);
 int kf_batch_launch_raycast(kf_batch* b, int n);
 
-// Zero the barrier counter and the ICP sum buffers of a state block before a tracking launch.
+// Zero the ICP reduction rows before a tracking launch.
 inline cudaError_t kf_clear_icp_words(KfDevState* st, cudaStream_t stream) {
-  const size_t b0 = offsetof(KfDevState, barrier_count);
-  const size_t b1 = offsetof(KfDevState, icp_acc) + sizeof(st->icp_acc);
-  return cudaMemsetAsync(reinterpret_cast<char*>(st) + b0, 0, b1 - b0, stream);
+  return cudaMemsetAsync(kf_icp_words(st), 0, KF_ICP_WORDS * 8, stream);
 }
 
 // Count kernels launched outside graph capture (captured graphs are counted per replay).

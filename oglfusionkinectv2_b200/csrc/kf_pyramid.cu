@@ -99,8 +99,8 @@ struct VNArgs {
   float mcx[3], mcy[3];     // invK[2][0], invK[2][1] per level (-cx_l/fx_l, -cy_l/fy_l)
   int mode;                 // 1 vertex, 2 normal from stored vertex, 3 both from depth
   int down_from_left;       // Q3
-  // frame step: the tracking launches that follow start from zeroed barrier counters and
-  // ICP sum buffers, which block 0 writes here (in place of two memset nodes)
+  // frame step: the tracking launches that follow start from a zero SDF barrier counter and
+  // zero ICP reduction rows, which block 0 writes here (in place of two memset nodes)
   KfDevState* clear_state;
 };
 
@@ -124,10 +124,8 @@ __global__ void __launch_bounds__(256) vertex_normal_kernel(VNArgs one, const VN
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   if (!BATCH && a.clear_state && blockIdx.x == 0) {
     KfDevState* st = a.clear_state;
-    if (threadIdx.x == 0) st->barrier_count = 0u;
     if (threadIdx.x == 1) st->sdf_barrier_count = 0u;
-    for (int k = threadIdx.x; k < (int)(sizeof(st->icp_acc) / sizeof(long long)); k += blockDim.x)
-      (&st->icp_acc[0][0][0])[k] = 0;
+    for (int k = threadIdx.x; k < KF_ICP_WORDS; k += blockDim.x) kf_icp_words(st)[k] = 0;
   }
   if (gid >= a.start[3]) return;
   const int l = gid < a.start[1] ? 0 : (gid < a.start[2] ? 1 : 2);

@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <type_traits>
 
 #include <atomic>
 
@@ -113,22 +114,7 @@ void free_all(kf_session* s) {
   free_mc(s);
   cudaFree(s->d_vol);
   cudaFree(s->d_bricks);
-  cudaFree(s->d_plan);
-  cudaFree(s->d_tiles);
-  cudaFree(s->d_depth_u16);
-  cudaFree(s->d_depth_f32_in);
-  for (int l = 0; l < 3; ++l) {
-    cudaFree(s->d_depth[l]);
-    cudaFree(s->d_vertex[l]);
-    cudaFree(s->d_normal[l]);
-    cudaFree(s->d_status[l]);
-  }
-  cudaFree(s->d_ref_vertex);
-  cudaFree(s->d_ref_normal);
-  cudaFree(s->d_sdf_rows);
-  cudaFree(s->d_partials);
-  cudaFree(s->d_state);
-  cudaFree(s->d_u32_scalar);
+  cudaFree(s->d_arena);
   cudaFree(s->d_mip);
   cudaFree(s->d_undistort_map);
   cudaFree(s->d_depth_prep);
@@ -136,13 +122,10 @@ void free_all(kf_session* s) {
   for (auto& e : s->head_ev)
     if (e) cudaEventDestroy(e);
   if (s->copy_stream) cudaStreamSynchronize(s->copy_stream);
-  cudaFree(s->d_frame_ring);
   for (auto& e : s->upload_ev)
     if (e) cudaEventDestroy(e);
   if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
   if (s->h_state) cudaFreeHost(s->h_state);
-  if (s->h_depth_pinned) cudaFreeHost(s->h_depth_pinned);
-  if (s->h_u32_scalar) cudaFreeHost(s->h_u32_scalar);
   for (auto& e : s->ev)
     if (e) cudaEventDestroy(e);
   for (auto& row : s->ring_ev)
@@ -218,7 +201,6 @@ int alloc_volume(kf_session* s) {
   cudaFree(s->d_bricks);
   s->d_bricks = nullptr;
   s->d_neg = nullptr;
-  cudaFree(s->d_plan);
   s->d_plan = nullptr;
   s->bx = (s->cfg.nx + KF_BRICK - 1) / KF_BRICK;
   s->by = (s->cfg.ny + KF_BRICK - 1) / KF_BRICK;
@@ -228,11 +210,13 @@ int alloc_volume(kf_session* s) {
   s->wz = (s->cfg.nz + KF_WORD - 1) / KF_WORD;
   {
     const size_t nb = (size_t)s->bx * s->by * s->bz;
-    int rc = dalloc(s, &s->d_bricks, kf_flag_words(s->bx, s->by, s->bz));
+    // one allocation: the flags, their bits, integrate's plan
+    const size_t flags = kf_flag_words(s->bx, s->by, s->bz);
+    int rc = dalloc(s, &s->d_bricks, flags + KF_PLAN_HEAD + nb);
     if (rc) return rc;
     s->d_neg = reinterpret_cast<unsigned long long*>(s->d_bricks + kf_brick_words(s->bx, s->by, s->bz));
     if ((rc = kf_reset_bricks(s))) return rc;
-    if ((rc = dalloc(s, &s->d_plan, KF_PLAN_HEAD + nb))) return rc;
+    s->d_plan = s->d_bricks + flags;
     KF_CUDA_TRY(s, cudaMemsetAsync(s->d_plan, 0, KF_PLAN_HEAD * 4, s->stream));
   }
   s->vol_count = (size_t)s->cfg.nx * s->cfg.ny * s->cfg.nz;
@@ -243,6 +227,46 @@ int alloc_volume(kf_session* s) {
   if (rc) return rc;
   s->d_vol = p;
   KF_CUDA_TRY(s, cudaMemsetAsync(s->d_vol, 0, s->vol_bytes, s->stream));
+  return KF_OK;
+}
+
+// Every buffer whose size depends on the image alone, in one zeroed allocation (an allocation
+// or a release costs up to a millisecond, whatever its size).
+int alloc_arena(kf_session* s) {
+  char* base = nullptr;
+  size_t used = 0;
+  auto take = [&](auto** p, size_t count) {
+    if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + used);
+    used += (count * sizeof(**p) + 255) & ~(size_t)255;
+  };
+  const size_t px = (size_t)s->W[0] * s->H[0];
+  char* state = nullptr;  // the control block, then the ICP reduction rows
+  auto layout = [&] {
+    used = 0;
+    take(&state, sizeof(KfDevState) + KF_ICP_WORDS * 8);
+    take(&s->d_u32_scalar, 4);
+    take(&s->d_depth_u16, px);
+    take(&s->d_frame_ring, px * kf_session::kRing);
+    take(&s->d_depth_f32_in, px);
+    for (int l = 0; l < 3; ++l) {
+      const size_t n = (size_t)s->W[l] * s->H[l];
+      take(&s->d_depth[l], n);
+      take(&s->d_vertex[l], n);
+      take(&s->d_normal[l], n);
+      take(&s->d_status[l], n);
+    }
+    take(&s->d_tiles, tile_count(s->W[0], s->H[0]));
+    take(&s->d_ref_vertex, px);
+    take(&s->d_ref_normal, px);
+    take(&s->d_sdf_rows, px * 8);
+    take(&s->d_partials, (size_t)2 * KF_MAX_TRACK_BLOCKS * 32);
+  };
+  layout();
+  if (int rc = dalloc(s, &base, used)) return rc;
+  s->d_arena = base;
+  layout();
+  s->d_state = reinterpret_cast<KfDevState*>(state);
+  KF_CUDA_TRY(s, cudaMemsetAsync(base, 0, used, s->stream));
   return KF_OK;
 }
 
@@ -569,38 +593,10 @@ int kf_create(const kf_config* cfg, const kf_intrinsics* intr, kf_session** out)
     s->W[l] = intr->width >> l;
     s->H[l] = intr->height >> l;
   }
-  const size_t px = (size_t)s->W[0] * s->H[0];
   if ((rc = alloc_volume(s))) return bail(rc);
-  if ((rc = dalloc(s, &s->d_depth_u16, px))) return bail(rc);
-  if ((rc = dalloc(s, &s->d_frame_ring, px * kf_session::kRing))) return bail(rc);
-  if ((rc = dalloc(s, &s->d_depth_f32_in, px))) return bail(rc);
-  for (int l = 0; l < 3; ++l) {
-    const size_t n = (size_t)s->W[l] * s->H[l];
-    if ((rc = dalloc(s, &s->d_depth[l], n))) return bail(rc);
-    if ((rc = dalloc(s, &s->d_vertex[l], n))) return bail(rc);
-    if ((rc = dalloc(s, &s->d_normal[l], n))) return bail(rc);
-    if ((rc = dalloc(s, &s->d_status[l], n))) return bail(rc);
-    cudaMemsetAsync(s->d_depth[l], 0, n * 4, s->stream);
-    cudaMemsetAsync(s->d_vertex[l], 0, n * 16, s->stream);
-    cudaMemsetAsync(s->d_normal[l], 0, n * 16, s->stream);
-    cudaMemsetAsync(s->d_status[l], 0, n * 4, s->stream);
-  }
-  if ((rc = dalloc(s, &s->d_tiles, tile_count(s->W[0], s->H[0])))) return bail(rc);
-  cudaMemsetAsync(s->d_tiles, 0, tile_count(s->W[0], s->H[0]) * 4, s->stream);
-  if ((rc = dalloc(s, &s->d_ref_vertex, px))) return bail(rc);
-  if ((rc = dalloc(s, &s->d_ref_normal, px))) return bail(rc);
-  if ((rc = dalloc(s, &s->d_sdf_rows, px * 8))) return bail(rc);
-  if ((rc = dalloc(s, &s->d_partials, (size_t)2 * KF_MAX_TRACK_BLOCKS * 32))) return bail(rc);
-  char* state = nullptr;  // the control block, then the ICP reduction rows
-  if ((rc = dalloc(s, &state, sizeof(KfDevState) + KF_ICP_WORDS * 8))) return bail(rc);
-  s->d_state = reinterpret_cast<KfDevState*>(state);
-  if ((rc = dalloc(s, &s->d_u32_scalar, 4))) return bail(rc);
-  cudaMemsetAsync(s->d_ref_vertex, 0, px * 16, s->stream);
-  cudaMemsetAsync(s->d_ref_normal, 0, px * 16, s->stream);
-  cudaMemsetAsync(s->d_sdf_rows, 0, px * 32, s->stream);
-  if (cudaMallocHost((void**)&s->h_state, sizeof(KfDevState)) != cudaSuccess) return bail(KF_ERR_OUT_OF_MEMORY);
-  if (cudaMallocHost((void**)&s->h_depth_pinned, px * 2) != cudaSuccess) return bail(KF_ERR_OUT_OF_MEMORY);
-  if (cudaMallocHost((void**)&s->h_u32_scalar, 16) != cudaSuccess) return bail(KF_ERR_OUT_OF_MEMORY);
+  if ((rc = alloc_arena(s))) return bail(rc);
+  if (cudaMallocHost((void**)&s->h_state, sizeof(KfDevState) + 16) != cudaSuccess) return bail(KF_ERR_OUT_OF_MEMORY);
+  s->h_u32_scalar = reinterpret_cast<uint32_t*>(s->h_state + 1);
   std::memset(s->h_state, 0, sizeof(KfDevState));
   kf_store_pose(s->h_state, kIdentity);
   std::memcpy(s->h_state->pose_eig, kIdentity, sizeof(kIdentity));

@@ -118,6 +118,9 @@ struct kf_session {
   size_t vol_value_bytes = 0;
   size_t vol_bytes = 0;
 
+  // one allocation for everything whose size depends on the image alone (the pointers below)
+  char* d_arena = nullptr;
+
   // image pyramid
   int W[3] = {0, 0, 0}, H[3] = {0, 0, 0};
   uint16_t* d_depth_u16 = nullptr;  // upload staging (device)
@@ -136,7 +139,6 @@ struct kf_session {
 
   KfDevState* d_state = nullptr;
   KfDevState* h_state = nullptr;  // pinned mirror
-  uint16_t* h_depth_pinned = nullptr;
 
   int track_blocks = 0;  // persistent grid of the tracking kernels
 
@@ -197,7 +199,7 @@ struct kf_session {
   uint32_t* d_mc_scratch = nullptr;  // level table / scan path verts, offsets, scan scratch
   size_t mc_scratch_words = 0;       // capacity of d_mc_scratch in bytes
   uint32_t* d_u32_scalar = nullptr;  // one device word for totals
-  uint32_t* h_u32_scalar = nullptr;  // pinned
+  uint32_t* h_u32_scalar = nullptr;  // pinned, after h_state
 
   float4* d_mip = nullptr;  // intensity-projection image, allocated on first use
 

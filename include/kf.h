@@ -143,7 +143,7 @@ typedef struct kf_volume_view {
   void* device_ptr;            /* value plane, for reading; valid until kf_reset(.., 1)  */
                                /* or kf_destroy.  New contents go in through            */
                                /* kf_copy_volume_from_host, which also refreshes the    */
-                               /* per-8^3-brick summary that kf_raycast skips by.       */
+                               /* per-8^3-brick flags by which the other calls skip.     */
   int32_t nx, ny, nz;
   int32_t storage;             /* KF_STORAGE_*                                           */
   int64_t value_bytes;         /* bytes per value (and per weight): 4 or 2              */

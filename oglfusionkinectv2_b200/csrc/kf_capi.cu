@@ -71,12 +71,9 @@ size_t tile_count(int w, int h) {
 size_t value_bytes(int storage) { return storage == KF_STORAGE_F32F32 ? 4 : 2; }
 
 void free_mc(kf_session* s) {
-  cudaFree(s->d_mc_base);
-  s->d_mc_base = nullptr;
-  for (uint32_t* p : s->d_mc_levels) cudaFree(p);
-  s->d_mc_levels.clear();
-  s->mc_P = 0;
-  s->mc_top = 0;
+  cudaFree(s->d_mc_cases);
+  s->d_mc_cases = nullptr;
+  s->mc_case_cap = 0;
   cudaFree(s->d_mc_vertices);
   s->d_mc_vertices = nullptr;
   s->mc_vertex_cap = 0;
@@ -88,14 +85,15 @@ void free_mc(kf_session* s) {
   s->mc_normal_cap = 0;
   s->mc_valid = 0;
   s->mc_triangles = 0;
-  cudaFree(s->d_mesh_mask);
+  cudaFree(s->d_mesh_cases);
   cudaFree(s->d_mesh_scratch);
   cudaFree(s->d_mesh_pos);
   cudaFree(s->d_mesh_nrm);
   cudaFree(s->d_mesh_idx);
-  s->d_mesh_mask = s->d_mesh_scratch = s->d_mesh_idx = nullptr;
+  s->d_mesh_cases = nullptr;
+  s->d_mesh_scratch = s->d_mesh_idx = nullptr;
   s->d_mesh_pos = s->d_mesh_nrm = nullptr;
-  s->mesh_mask_cap = s->mesh_scratch_cap = s->mesh_pos_cap = s->mesh_nrm_cap = s->mesh_idx_cap = 0;
+  s->mesh_case_cap = s->mesh_scratch_cap = s->mesh_pos_cap = s->mesh_nrm_cap = s->mesh_idx_cap = 0;
   s->mesh_vertices = s->mesh_triangles = 0;
   s->mesh_valid = 0;
 }

@@ -176,17 +176,16 @@ struct kf_session {
   bool capturing = false;
 
   // marching cubes
-  uint32_t* d_mc_base = nullptr;  // nx*ny*nz cubes: numTri | cubeIndex << 16
-  std::vector<uint32_t*> d_mc_levels;  // level k >= 1, (P >> k)^3
-  int mc_P = 0, mc_top = 0;
+  uint8_t* d_mc_cases = nullptr;  // case index per cube of the last extraction's listed tiles, their list
+  size_t mc_case_cap = 0;
   float4* d_mc_vertices = nullptr;
   size_t mc_vertex_cap = 0;
   float4* d_mc_normals = nullptr;  // face normal of each soup vertex's triangle (w = 0)
   size_t mc_normal_cap = 0;
   // welded mesh (kf_mc_extract_mesh): one vertex per cut voxel edge, indexed triangles
-  uint32_t* d_mesh_mask = nullptr;  // edge bits, 10 voxels x 3 axes per word
-  size_t mesh_mask_cap = 0;
-  uint32_t* d_mesh_scratch = nullptr;  // triangle counts/offsets, word offsets, scan scratch
+  uint8_t* d_mesh_cases = nullptr;
+  size_t mesh_case_cap = 0;
+  uint32_t* d_mesh_scratch = nullptr;  // counts, edge marks, offsets, scan scratch
   size_t mesh_scratch_cap = 0;
   float* d_mesh_pos = nullptr;  // 3 floats per vertex (metres)
   float* d_mesh_nrm = nullptr;  // 3 floats per vertex (unit)
@@ -196,7 +195,7 @@ struct kf_session {
   int mesh_valid = 0;
   uint32_t mc_triangles = 0;
   int mc_valid = 0;
-  uint32_t* d_mc_scratch = nullptr;  // level table / scan path verts, offsets, scan scratch
+  uint32_t* d_mc_scratch = nullptr;  // counts, offsets, scan scratch
   size_t mc_scratch_words = 0;       // capacity of d_mc_scratch in bytes
   uint32_t* d_u32_scalar = nullptr;  // one device word for totals
   uint32_t* h_u32_scalar = nullptr;  // pinned, after h_state

@@ -211,3 +211,40 @@ def test_welded_mesh_matches_oracle(storage, tmp_path):
     c = np.array([0.5, 0.5, 0.5])
     cen = Pg[Ig].mean(axis=1)
     assert np.mean(np.sum(fn * (cen - c), axis=1) > 0) > 0.999  # outward facets
+
+
+@pytest.mark.parametrize("size", [(33, 41, 47), (64, 24, 9), (131, 60, 57)])
+@pytest.mark.parametrize("storage,iso", [(L.KF_STORAGE_F32F32, 0.25), (L.KF_STORAGE_F16U16, -0.25), (L.KF_STORAGE_RG16I, 9000.0)])
+def test_ragged_tiles_and_levels(size, storage, iso):
+    """Volumes that end inside a tile, a level above zero (every tile is looked at) and one
+    below; then a larger surface in the same session, whose triangles the first one's buffer
+    cannot hold.  Two blobs of other sizes, so that most tiles are empty.  The case bytes come
+    from comparisons alone, so they and all counts are equal; positions as in compare()."""
+    nx, ny, nz = size
+    cfg = GFusionConfig(volumeSize=size, volumeDimensions=tuple(n / 100.0 for n in size), storage=storage,
+                        quirks=L.KF_QUIRKS_TRACKING & ~(L.KF_Q13_MC_FIRST_SEVEN | L.KF_Q15_MC_BORDER_SKIP))
+    Z, Y, X = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+
+    def raw(r):
+        sd = np.minimum(np.sqrt((X - nx * 0.8) ** 2 + (Y - ny * 0.7) ** 2 + (Z - nz * 0.5) ** 2) - r,
+                        np.sqrt((X - 4.3) ** 2 + (Y - 5.1) ** 2 + (Z - 4.4) ** 2) - r / 2)
+        F = np.clip(sd / 6.0, -1, 1).astype(np.float32).ravel()
+        W = np.ones(F.size, np.float32)
+        if storage == L.KF_STORAGE_F32F32:
+            return np.concatenate([F, W]).view(np.uint8)
+        if storage == L.KF_STORAGE_RG16I:
+            return np.concatenate([(F * 32766).astype(np.int32).astype(np.int16), W.astype(np.int16)]).view(np.uint8)
+        return np.concatenate([F.astype(np.float16).view(np.uint16), W.astype(np.uint16)]).view(np.uint8)
+
+    g, o = both(cfg, raw(3.6))
+    for blob in (3.6, 0.45 * min(size) + 3.0):
+        g.setVolumeRaw(raw(blob))
+        o.setVolumeRaw(raw(blob))
+        for method in (L.KF_MC_HISTOPYRAMID, L.KF_MC_SCAN):
+            m, n = compare(g, o, method, iso)
+            assert n > 0
+        Pg, Ng, Ig = m.extractMesh()
+        Po, No, Io = o.mcMesh(iso)
+        assert len(Pg) == len(Po)
+        np.testing.assert_array_equal(Ig, Io)
+        assert np.max(np.abs(Pg - Po)) <= 1e-6

@@ -485,7 +485,8 @@ KF_API int kf_prefix_sum_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, 
 /* Allocation-free prefix sum.  No counterpart in the reference: it exists for callers that
  * must not allocate device memory, such as a frame loop running under a fixed memory
  * budget or inside a host framework that owns every device allocation, where the
- * cudaMalloc of kf_prefix_sum_u32's scratch is not allowed.  Same result as
+ * scratch that kf_prefix_sum_u32 allocates for more than 2^28 elements, or when many threads
+ * call it at once, is not allowed.  Same result as
  * kf_prefix_sum_u32; the scratch is a 262,220-byte array compiled into the library,
  * which every GPU that loads the library keeps until the process exits.
  *   - n may be at most 2^28 (268,435,456) elements; larger n returns KF_ERR_CAPACITY.

@@ -960,8 +960,9 @@ inline size_t kf_flag_words(int bx, int by, int bz) {
 }
 #define KF_BRICK_REBUILD_EVERY 16
 int kf_mc_run(kf_session* s, float iso, int method, uint32_t* n_tri);
-int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, uint32_t* d_total,
-                cudaStream_t stream, uint32_t* d_scratch, size_t scratch_words);
+// *result: two device words in the scratch, the total and (not 0) that a wait gave up.
+int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, cudaStream_t stream, uint32_t* d_scratch,
+                size_t scratch_words, const uint32_t** result);
 size_t kf_scan_scratch_words(uint64_t n);
 // Co-resident blocks of `kernel` on the session's device: min(per SM, max_per_sm) x SMs
 // (with the default 2, capped at KF_MAX_TRACK_BLOCKS for the tracking kernels).

@@ -644,7 +644,8 @@ McArgs make_mc_args(kf_session* s, float iso) {
 
 size_t tile_count(const McArgs& a) { return (size_t)a.tx * a.ty * a.tz; }
 
-size_t segment_count(const McArgs& a) { return (size_t)a.tx * a.ny * a.nz; }
+// rounded up, so that the arrays of that many words behind one another are 16-byte aligned
+size_t segment_count(const McArgs& a) { return ((size_t)a.tx * a.ny * a.nz + 3) & ~(size_t)3; }
 
 #define KF_MC_LAUNCH(kernel, grid, threads, ...)                                                             \
   do {                                                                                                       \
@@ -694,6 +695,20 @@ int walk_blocks(const kf_session* s) { return 6 * s->num_sms; }
 int gen_blocks(const kf_session* s) { return 16 * s->num_sms; }  // 512^3: 104, 74, 73, 64 us at 4, 8, 12, 16
 constexpr int kGenThreads = 32 * kGenWarps;
 
+// Prefix sum of the counts; its result is on the way to two pinned words.
+int scan_counts(kf_session* s, const uint32_t* counts, uint32_t* offsets, uint64_t n, uint32_t* scratch, size_t words,
+                uint32_t* host) {
+  const uint32_t* result = nullptr;
+  if (int rc = kf_scan_u32(counts, offsets, n, s->stream, scratch, words, &result)) return rc;
+  KF_CUDA_TRY(s, cudaMemcpyAsync(host, result, 8, cudaMemcpyDeviceToHost, s->stream));
+  return KF_OK;
+}
+int scan_check(kf_session* s, const uint32_t* host) {
+  if (!host[1]) return KF_OK;
+  s->last_error = "prefix sum: a wait for another block gave up";
+  return KF_ERR_CUDA;
+}
+
 int histopyramid(kf_session* s, float iso, uint32_t* n_tri) {
   McArgs a = make_mc_args(s, iso);
   uint32_t side = 1;  // bricks per side of the pyramid's power-of-two cube
@@ -703,25 +718,24 @@ int histopyramid(kf_session* s, float iso, uint32_t* n_tri) {
   int rc;
   // case bytes, then the list of their tiles
   if ((rc = ensure(s, (void**)&s->d_mc_cases, &s->mc_case_cap, tile_count(a) * kTileCubes + list_words(a) * 4))) return rc;
-  // counts[codes], offsets[codes], scan scratch, total
-  if ((rc = ensure(s, (void**)&s->d_mc_scratch, &s->mc_scratch_words, (2 * (size_t)codes + sw + 1) * 4))) return rc;
+  // counts[codes], offsets[codes], scan scratch
+  if ((rc = ensure(s, (void**)&s->d_mc_scratch, &s->mc_scratch_words, (2 * (size_t)codes + sw) * 4))) return rc;
   uint32_t* offs = s->d_mc_scratch + codes;
-  uint32_t* total = offs + codes + sw;
   a.cases = s->d_mc_cases;
   a.counts = s->d_mc_scratch;
   a.offsets = offs;
   KF_CUDA_TRY(s, cudaMemsetAsync(a.counts, 0, (size_t)codes * 4, s->stream));
   if ((rc = list_tiles(s, &a, case_tiles(s, a)))) return rc;
   KF_MC_LAUNCH(histo_classify_kernel, walk_blocks(s), 256, a);
-  if ((rc = kf_scan_u32(a.counts, offs, codes, total, s->stream, offs + codes, sw))) return rc;
-  // the triangle count (glGetTexImage of the top texel at mcubes.cpp:290-300)
-  KF_CUDA_TRY(s, cudaMemcpyAsync(s->h_u32_scalar, total, 4, cudaMemcpyDeviceToHost, s->stream));
+  // and the triangle count (glGetTexImage of the top texel at mcubes.cpp:290-300)
+  if ((rc = scan_counts(s, a.counts, offs, codes, offs + codes, sw, s->h_u32_scalar))) return rc;
   for (;;) {
     a.cap = soup_capacity(s) / 3;
     a.out = s->d_mc_vertices;
     a.nout = s->d_mc_normals;
     if (a.out && a.nout) KF_MC_LAUNCH(histo_generate_kernel, gen_blocks(s), kGenThreads, a);
     KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    if ((rc = scan_check(s, s->h_u32_scalar))) return rc;
     const uint32_t T = s->h_u32_scalar[0];
     if (a.out && a.nout && T <= a.cap) {
       *n_tri = T;
@@ -738,10 +752,9 @@ int classic(kf_session* s, float iso, uint32_t* n_tri) {
   int rc;
   // case bytes, then the list of their tiles
   if ((rc = ensure(s, (void**)&s->d_mc_cases, &s->mc_case_cap, tile_count(a) * kTileCubes + list_words(a) * 4))) return rc;
-  // counts[n], offsets[n], scan scratch, total
-  if ((rc = ensure(s, (void**)&s->d_mc_scratch, &s->mc_scratch_words, (2 * n + sw + 1) * 4))) return rc;
+  // counts[n], offsets[n], scan scratch
+  if ((rc = ensure(s, (void**)&s->d_mc_scratch, &s->mc_scratch_words, (2 * n + sw) * 4))) return rc;
   uint32_t* offs = s->d_mc_scratch + n;
-  uint32_t* total = offs + n + sw;
   a.cases = s->d_mc_cases;
   a.counts = s->d_mc_scratch;
   a.offsets = offs;
@@ -752,14 +765,14 @@ int classic(kf_session* s, float iso, uint32_t* n_tri) {
   KF_CUDA_TRY(s, cudaMemsetAsync(a.counts, 0, n * 4, s->stream));
   if ((rc = list_tiles(s, &a, case_tiles(s, a)))) return rc;
   KF_MC_LAUNCH(classic_classify_kernel, walk_blocks(s), 256, a);
-  if ((rc = kf_scan_u32(a.counts, offs, n, total, s->stream, offs + n, sw))) return rc;
-  KF_CUDA_TRY(s, cudaMemcpyAsync(s->h_u32_scalar, total, 4, cudaMemcpyDeviceToHost, s->stream));
+  if ((rc = scan_counts(s, a.counts, offs, n, offs + n, sw, s->h_u32_scalar))) return rc;
   for (;;) {
     a.cap = soup_capacity(s);
     a.out = s->d_mc_vertices;
     a.nout = s->d_mc_normals;
     if (a.out && a.nout) KF_MC_LAUNCH(classic_generate_kernel, gen_blocks(s), kGenThreads, a);
     KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    if ((rc = scan_check(s, s->h_u32_scalar))) return rc;
     const uint32_t nverts = s->h_u32_scalar[0];
     if (a.out && a.nout && nverts <= a.cap) {
       *n_tri = nverts / 3;
@@ -786,10 +799,10 @@ int extract_mesh(kf_session* s, float iso, uint32_t* nv_out, uint32_t* nt_out) {
   int rc;
   if ((rc = ensure(s, (void**)&s->d_mesh_cases, &s->mesh_case_cap, tile_count(a) * kTileCubes))) return rc;
   // triangles[n], vertices[n], edge marks[3 n], triangle offsets[n], vertex offsets[n], scan
-  // scratch, 2 totals, tile list
-  if ((rc = ensure(s, (void**)&s->d_mesh_scratch, &s->mesh_scratch_cap, (7 * n + sw + 2 + list_words(a)) * 4))) return rc;
+  // scratch twice, tile list
+  if ((rc = ensure(s, (void**)&s->d_mesh_scratch, &s->mesh_scratch_cap, (7 * n + 2 * sw + list_words(a)) * 4))) return rc;
   uint32_t* w = s->d_mesh_scratch;
-  uint32_t *toff = w + 5 * n, *voff = w + 6 * n, *scr = w + 7 * n, *totals = scr + sw;
+  uint32_t *toff = w + 5 * n, *voff = w + 6 * n, *scr = w + 7 * n;
   a.cases = s->d_mesh_cases;
   a.counts = w;
   a.vcounts = w + n;
@@ -797,14 +810,13 @@ int extract_mesh(kf_session* s, float iso, uint32_t* nv_out, uint32_t* nt_out) {
   a.offsets = toff;
   a.voffsets = voff;
   KF_CUDA_TRY(s, cudaMemsetAsync(w, 0, 5 * n * 4, s->stream));
-  if ((rc = list_tiles(s, &a, totals + 2))) return rc;
+  if ((rc = list_tiles(s, &a, scr + 2 * sw))) return rc;
   KF_MC_LAUNCH(mesh_mark_kernel, walk_blocks(s), 256, a);
   mesh_count_kernel<<<walk_blocks(s), 256, 0, s->stream>>>(a);
   KF_CUDA_TRY(s, cudaGetLastError());
   kf_note_launch(s);
-  if ((rc = kf_scan_u32(a.counts, toff, n, totals, s->stream, scr, sw))) return rc;
-  if ((rc = kf_scan_u32(a.vcounts, voff, n, totals + 1, s->stream, scr, sw))) return rc;
-  KF_CUDA_TRY(s, cudaMemcpyAsync(s->h_u32_scalar, totals, 8, cudaMemcpyDeviceToHost, s->stream));
+  if ((rc = scan_counts(s, a.counts, toff, n, scr, sw, s->h_u32_scalar))) return rc;
+  if ((rc = scan_counts(s, a.vcounts, voff, n, scr + sw, sw, s->h_u32_scalar + 2))) return rc;
   for (;;) {
     // launched for what the buffers hold, and again if that was too little
     a.vcap = (uint32_t)std::min<size_t>(std::min(s->mesh_pos_cap, s->mesh_nrm_cap) / 12, 0xffffffffu);
@@ -819,7 +831,8 @@ int extract_mesh(kf_session* s, float iso, uint32_t* nv_out, uint32_t* nt_out) {
       kf_note_launch(s);
     }
     KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-    const uint32_t T = s->h_u32_scalar[0], NV = s->h_u32_scalar[1];
+    if ((rc = scan_check(s, s->h_u32_scalar)) || (rc = scan_check(s, s->h_u32_scalar + 2))) return rc;
+    const uint32_t T = s->h_u32_scalar[0], NV = s->h_u32_scalar[2];
     if ((uint64_t)T * 3 >= (1ull << 32)) return KF_ERR_CAPACITY;
     if (NV <= a.vcap && T <= a.cap) {
       s->mesh_vertices = NV;

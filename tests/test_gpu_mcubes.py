@@ -248,3 +248,64 @@ def test_ragged_tiles_and_levels(size, storage, iso):
         assert len(Pg) == len(Po)
         np.testing.assert_array_equal(Ig, Io)
         assert np.max(np.abs(Pg - Po)) <= 1e-6
+
+
+@pytest.mark.parametrize("shift_in,shift_out", [(0, 0), (3, 3), (1, 0), (0, 2)])
+def test_prefix_sum_tiles_and_alignment(shift_in, shift_out):
+    """Both sides of a tile's and a look-back window's end, inputs and outputs that start off a
+    16-byte boundary, in place, and nothing written outside [0, n).  Integers: exact."""
+    import torch
+    lib = L.load()
+    rng = np.random.default_rng(5)
+    T = 16384
+    for n in (1, 2, 5, T - 4, T - 1, T, T + 1, 3 * T + 2, 148 * T - 3, 161 * T + 7, 460 * T + 1):
+        a = rng.integers(0, 2 ** 20, n, dtype=np.uint32)
+        ref, rtot = O.prefix_sum(a)
+        guard = np.full(n + 16, 0xABCDEF01, np.uint32)
+        src = guard.copy()
+        src[shift_in:shift_in + n] = a
+        d_in = torch.from_numpy(src.view(np.int32)).cuda()
+        for fn in (lib.kf_prefix_sum_u32, lib.kf_prefix_sum_u32_noalloc):
+            d_out = torch.from_numpy(guard.view(np.int32)).cuda()
+            tot = C.c_uint32()
+            assert fn(C.c_void_p(d_in.data_ptr() + 4 * shift_in), C.c_void_p(d_out.data_ptr() + 4 * shift_out), n,
+                      C.byref(tot), None) == L.KF_OK
+            out = d_out.cpu().numpy().view(np.uint32)
+            np.testing.assert_array_equal(out[shift_out:shift_out + n], ref)
+            assert tot.value == rtot
+            assert (np.delete(out, np.s_[shift_out:shift_out + n]) == 0xABCDEF01).all()
+        p = C.c_void_p(d_in.data_ptr() + 4 * shift_in)
+        assert lib.kf_prefix_sum_u32(p, p, n, None, None) == L.KF_OK
+        np.testing.assert_array_equal(d_in.cpu().numpy().view(np.uint32)[shift_in:shift_in + n], ref)
+
+
+@pytest.mark.parametrize("threads", [2, 7])
+def test_prefix_sums_of_several_threads(threads):
+    """Calls at once on streams of their own, also more than there are slots of scratch."""
+    import threading
+    import torch
+    lib = L.load()
+    wrong = []
+
+    def work(k):
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            n = 200_000 + 17 * k
+            x = torch.full((n,), k + 1, dtype=torch.int32, device="cuda")
+            o = torch.empty_like(x)
+            expect = torch.arange(n, dtype=torch.int32, device="cuda") * (k + 1)
+            st.synchronize()
+            for _ in range(20):
+                o.fill_(-1)
+                tot = C.c_uint32()
+                rc = lib.kf_prefix_sum_u32(C.c_void_p(x.data_ptr()), C.c_void_p(o.data_ptr()), n, C.byref(tot),
+                                           C.c_void_p(st.cuda_stream))
+                if rc != L.KF_OK or tot.value != n * (k + 1) or not torch.equal(o, expect):
+                    wrong.append((k, rc, tot.value))
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(threads)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not wrong

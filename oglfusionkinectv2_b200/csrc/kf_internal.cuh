@@ -959,6 +959,8 @@ inline size_t kf_flag_words(int bx, int by, int bz) {
   return kf_brick_words(bx, by, bz) + 2 * (size_t)((bx + 3) / 4) * ((by + 3) / 4) * ((bz + 3) / 4);
 }
 #define KF_BRICK_REBUILD_EVERY 16
+// Device to host memory of the caller's; returns when it is there.
+int kf_copy_to_host(kf_session* s, void* dst, const void* src, size_t bytes);
 int kf_mc_run(kf_session* s, float iso, int method, uint32_t* n_tri);
 // *result: two device words in the scratch, the total and (not 0) that a wait gave up.
 int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, cudaStream_t stream, uint32_t* d_scratch,

@@ -891,9 +891,7 @@ int kf_mc_copy_vertices(kf_session* s, float* v, uint64_t max_vertices) {
   const uint64_t n = (uint64_t)s->mc_triangles * 3;
   if (max_vertices < n) return KF_ERR_CAPACITY;
   if (!n) return KF_OK;
-  KF_CUDA_TRY(s, cudaMemcpyAsync(v, s->d_mc_vertices, n * 16, cudaMemcpyDeviceToHost, s->stream));
-  KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-  return KF_OK;
+  return kf_copy_to_host(s, v, s->d_mc_vertices, n * 16);
 }
 
 int kf_mc_copy_normals(kf_session* s, float* n4, uint64_t max_vertices) {
@@ -902,9 +900,7 @@ int kf_mc_copy_normals(kf_session* s, float* n4, uint64_t max_vertices) {
   const uint64_t n = (uint64_t)s->mc_triangles * 3;
   if (max_vertices < n) return KF_ERR_CAPACITY;
   if (!n) return KF_OK;
-  KF_CUDA_TRY(s, cudaMemcpyAsync(n4, s->d_mc_normals, n * 16, cudaMemcpyDeviceToHost, s->stream));
-  KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-  return KF_OK;
+  return kf_copy_to_host(s, n4, s->d_mc_normals, n * 16);
 }
 
 int kf_mc_copy_base_level(kf_session* s, uint32_t* base, uint64_t count) {
@@ -987,11 +983,11 @@ int kf_mc_copy_mesh(kf_session* s, float* positions3, float* normals3, uint32_t*
   const uint64_t nv = s->mesh_vertices, nt = s->mesh_triangles;
   if (max_vertices < nv || max_triangles < nt) return KF_ERR_CAPACITY;
   if ((nv && (!positions3 && !normals3)) || (nt && !indices3 && !positions3 && !normals3)) return KF_ERR_INVALID_ARGUMENT;
-  if (nv && positions3) KF_CUDA_TRY(s, cudaMemcpyAsync(positions3, s->d_mesh_pos, nv * 12, cudaMemcpyDeviceToHost, s->stream));
-  if (nv && normals3) KF_CUDA_TRY(s, cudaMemcpyAsync(normals3, s->d_mesh_nrm, nv * 12, cudaMemcpyDeviceToHost, s->stream));
-  if (nt && indices3) KF_CUDA_TRY(s, cudaMemcpyAsync(indices3, s->d_mesh_idx, nt * 12, cudaMemcpyDeviceToHost, s->stream));
-  KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-  return KF_OK;
+  int rc = KF_OK;
+  if (nv && positions3) rc = kf_copy_to_host(s, positions3, s->d_mesh_pos, nv * 12);
+  if (!rc && nv && normals3) rc = kf_copy_to_host(s, normals3, s->d_mesh_nrm, nv * 12);
+  if (!rc && nt && indices3) rc = kf_copy_to_host(s, indices3, s->d_mesh_idx, nt * 12);
+  return rc;
 }
 
 int kf_mc_export_mesh_ply(kf_session* s, const char* path) {

@@ -144,3 +144,25 @@ def test_non_finite_poses_are_rejected():
                 call(p)
             assert e.value.status == L.KF_ERR_INVALID_ARGUMENT
     np.testing.assert_array_equal(g.getPose(), before)
+
+
+@pytest.mark.parametrize("voxels", [(64, 64, 63), (64, 64, 64), (131, 127, 129)])
+def test_copy_into_untouched_memory(voxels):
+    """Copies to host memory that nothing has written yet, just below and above the size from which
+    its pages are mapped ahead, at an odd address; the bytes around the destination keep theirs."""
+    import ctypes as C
+    import mmap
+    from oglfusionkinectv2_b200 import GFusionConfig, Intrinsics
+    g = GFusion(GFusionConfig(volumeSize=voxels, volumeDimensions=(1.0,) * 3, storage=L.KF_STORAGE_F16U16), Intrinsics())
+    n = int(np.prod(voxels)) * 4
+    raw = np.random.default_rng(3).integers(0, 255, n, dtype=np.uint8)
+    g.setVolumeRaw(raw)
+    for off in (0, 4099):
+        mm = mmap.mmap(-1, n + 3 * 4096, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        buf = np.frombuffer(mm, np.uint8)
+        if off:
+            buf[off - 1] = 77
+            buf[off + n] = 78
+        assert g.lib.kf_copy_volume_to_host(g._h, C.c_void_p(buf.ctypes.data + off), n) == L.KF_OK
+        np.testing.assert_array_equal(buf[off:off + n], raw)
+        assert off == 0 or (buf[off - 1] == 77 and buf[off + n] == 78)

@@ -359,20 +359,27 @@ __host__ __device__ inline void kf_se3_exp(const double* xi, double* T) {
   // [w]x column-major
   const double W[9] = {0, w2, -w1, -w2, 0, w0, w1, -w0, 0};
   double W2[9];
+#pragma unroll
   for (int c = 0; c < 3; ++c)
+#pragma unroll
     for (int r = 0; r < 3; ++r) {
       double s = 0;
+#pragma unroll
       for (int k = 0; k < 3; ++k) s += W[k * 3 + r] * W[c * 3 + k];
       W2[c * 3 + r] = s;
     }
   double R[9], V[9];
+#pragma unroll
   for (int i = 0; i < 9; ++i) {
     double I = (i % 4 == 0) ? 1.0 : 0.0;
     R[i] = I + A * W[i] + B * W2[i];
     V[i] = I + B * W[i] + C * W2[i];
   }
+#pragma unroll
   for (int c = 0; c < 3; ++c)
+#pragma unroll
     for (int r = 0; r < 3; ++r) T[c * 4 + r] = R[c * 3 + r];
+#pragma unroll
   for (int r = 0; r < 3; ++r) T[12 + r] = V[r] * xi[3] + V[3 + r] * xi[4] + V[6 + r] * xi[5];
   T[3] = T[7] = T[11] = 0;
   T[15] = 1;
@@ -391,29 +398,40 @@ __host__ __device__ inline void kf_store_pose(KfDevState* st, const double* P) {
 }
 
 // LDL^T solve (C.ldlt().solve(b), gFusion.cpp:902), unpivoted; NaN in, NaN out.
+// Unrolled, so that the matrix stays in registers on the device.
 __host__ __device__ inline void kf_ldlt6(const double* C, const double* b, double* x) {
   double L[36], D[6];
+#pragma unroll
   for (int i = 0; i < 36; ++i) L[i] = 0;
+#pragma unroll
   for (int j = 0; j < 6; ++j) {
     double d = C[j * 7];
+#pragma unroll
     for (int k = 0; k < j; ++k) d -= L[j * 6 + k] * L[j * 6 + k] * D[k];
     D[j] = d;
     L[j * 7] = 1;
+#pragma unroll
     for (int i = j + 1; i < 6; ++i) {
       double v = C[i * 6 + j];
+#pragma unroll
       for (int k = 0; k < j; ++k) v -= L[i * 6 + k] * L[j * 6 + k] * D[k];
       L[i * 6 + j] = v / d;
     }
   }
   double y[6];
+#pragma unroll
   for (int i = 0; i < 6; ++i) {
     double v = b[i];
+#pragma unroll
     for (int k = 0; k < i; ++k) v -= L[i * 6 + k] * y[k];
     y[i] = v;
   }
+#pragma unroll
   for (int i = 0; i < 6; ++i) y[i] /= D[i];
+#pragma unroll
   for (int i = 5; i >= 0; --i) {
     double v = y[i];
+#pragma unroll
     for (int k = i + 1; k < 6; ++k) v -= L[k * 6 + i] * x[k];
     x[i] = v;
   }
@@ -422,7 +440,9 @@ __host__ __device__ inline void kf_ldlt6(const double* C, const double* b, doubl
 // makeJTJ (gFusion.h:472-487): symmetric 6x6 from the 21 upper-triangular sums.
 __host__ __device__ inline void kf_make_jtj(const double* v21, double* C) {
   int k = 0;
+#pragma unroll
   for (int i = 0; i < 6; ++i)
+#pragma unroll
     for (int j = i; j < 6; ++j) {
       C[i * 6 + j] = v21[k];
       C[j * 6 + i] = v21[k];

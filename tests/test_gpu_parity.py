@@ -413,3 +413,20 @@ def test_icp_plane_only_rank_guard(jtj):
                 k += 1
         lam = np.linalg.eigvalsh(Cm)
         assert lam[2] < 1e-5 * lam[-1] and lam[3] > 1e-3 * lam[-1], lam
+
+
+@pytest.mark.parametrize("storage", [L.KF_STORAGE_F32F32, L.KF_STORAGE_F16U16, L.KF_STORAGE_RG16I])
+@pytest.mark.parametrize("size,dims", [((96, 80, 72), (1.5, 1.25, 1.125)), ((40, 40, 40), (3.0, 3.0, 3.0))])
+def test_sdf_taps_at_the_volume_edge(storage, size, dims):
+    """SDF tracking in volumes so small that many points and their neighbours fall outside, beside
+    points whose taps are shared: the oracle looks every tap up by itself.  Same bounds as the
+    teacher-forced test."""
+    w = small_workload(4, size=64, tracking=L.KF_TRACK_SDF, storage=storage)
+    w.config.volumeSize = size
+    w.config.volumeDimensions = dims
+    for k in (1, 2):
+        g, o, tg, to = _teacher_forced(w, k, "TrackSDF")
+        assert tg == to
+        Pg, Po = g.getPose(), o.getPose()
+        assert np.linalg.norm(Pg[:3, 3] - Po[:3, 3]) <= 1e-4
+        assert rot_deg(Pg, Po) <= 0.01

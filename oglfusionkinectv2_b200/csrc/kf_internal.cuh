@@ -79,7 +79,7 @@ static_assert(KF_STATE_RESULT_BYTES == 144, "frame result head: pose, tracked, e
 // Where the autotuner's timing launches write instead of the session's own buffers.
 struct kf_scratch_target {
   void* vol;             // integrate: a copy of the volume
-  uint32_t* bricks;      // and of the brick / super-brick flags
+  uint32_t* bricks;      // and of the brick flags
   unsigned long long* neg;
   float4* out_v;         // raycast: vertex and normal maps
   float4* out_n;
@@ -815,7 +815,7 @@ struct kf_batch {
   KfDevState* const* states = nullptr;
   const void* pyr_args = nullptr;
   const void* vn_args = nullptr;
-  int vn_pixels = 0, W1 = 0, H1 = 0;
+  int vn_tiles = 0, W1 = 0, H1 = 0;
   const void* icp_args = nullptr;
   int icp_blocks = 0;
   // the batched ICP runs in waves of at most KF_BATCH_ICP_WAVE members, each wave one

@@ -9,7 +9,7 @@ import pytest
 
 import kf_oracle as O
 from helpers import integrate_ambiguous, raycast_ambiguous, rot_deg, small_workload
-from oglfusionkinectv2_b200 import GFusion, synth, _lib as L
+from oglfusionkinectv2_b200 import GFusion, GFusionConfig, Intrinsics, synth, _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -430,3 +430,29 @@ def test_sdf_taps_at_the_volume_edge(storage, size, dims):
         Pg, Po = g.getPose(), o.getPose()
         assert np.linalg.norm(Pg[:3, 3] - Po[:3, 3]) <= 1e-4
         assert rot_deg(Pg, Po) <= 0.01
+
+
+@pytest.mark.parametrize("wh", [(16, 16), (36, 20), (132, 100)])
+@pytest.mark.parametrize("quirks", ["tracking", "reference"])
+def test_vertex_normal_tiles(wh, quirks):
+    """Images that end inside a 32 x 8 tile on every level, with holes: the frame step's launch
+    (normals from depth) and the separate one (from the stored vertices) give the same bits, and
+    the oracle's values within test_pyramid_parity's bounds."""
+    w, h = wh
+    intr = Intrinsics(width=w, height=h, fx=0.7 * w, fy=0.7 * w, cx=w / 2, cy=h / 2)
+    cfg = GFusionConfig(volumeSize=(32, 32, 32), volumeDimensions=(2.0, 2.0, 2.0), quirks=QUIRKS[quirks])
+    rng = np.random.default_rng(w)
+    f = (900 + 40 * np.sin(np.arange(w) / 5)[None, :] + 30 * np.cos(np.arange(h) / 3)[:, None] + rng.integers(0, 9, (h, w)))
+    f = np.where(rng.random((h, w)) < 0.05, 0, f).astype(np.uint16)
+    g, o = GFusion(cfg, intr), O.Oracle(cfg, intr)
+    for s in (g, o):
+        s.depthToVertex(f)
+        s.vertexToNormal()
+    k = GFusion(cfg, intr)
+    k.frameStep(f)
+    for l in range(3):
+        Vg, Ng, No = g.getVertexMap(l), g.getNormalMap(l), o.getNormalMap(l)
+        np.testing.assert_array_equal(k.getVertexMap(l), Vg)
+        np.testing.assert_array_equal(k.getNormalMap(l), Ng)
+        assert np.max(np.abs(Vg[..., :3] - o.getVertexMap(l)[..., :3])) < 2e-6
+        np.testing.assert_array_equal(Ng[..., 0] == 2, No[..., 0] == 2)

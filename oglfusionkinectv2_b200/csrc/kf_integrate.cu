@@ -367,20 +367,20 @@ __device__ __forceinline__ void integrate_half_brick(const IntArgs& a, uint32_t 
   }
 }
 
-// Small volumes: every warp tests one brick and runs it at once, which saves the list and a
+// Small volumes: every warp tests one brick and runs it, or (split 1) half of it, at once, which saves the list and a
 // launch.  A warp's test costs about as many instructions as half a brick's voxels, all lanes
 // doing the same, so it pays only while the launches' latency dominates (see kSmallBricks).
 template <int S>
-__global__ void __launch_bounds__(256, 4) integrate_small_kernel(IntArgs a) {
+__global__ void __launch_bounds__(256, 4) integrate_small_kernel(IntArgs a, int split) {
   if (a.gate && *(volatile const int*)a.gate == 0) return;
-  const int lane = threadIdx.x & 31, b = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, w = blockIdx.x * 8 + (threadIdx.x >> 5), b = w >> split;
   if (b >= a.bx * a.by * a.bz) return;
   const int bx = b % a.bx, by = b / a.bx % a.by, bz = b / (a.bx * a.by);
   const uint32_t word = a.bricks[b];
   if (!brick_changes(a, a.st->inv_rows, bx, by, bz, word)) return;
   const uint32_t entry = entry_of(bx, by, bz) | (word & KF_BRICK_SET ? kEntrySet : 0u);
 #pragma unroll 1
-  for (int half = 0; half < 2; ++half) integrate_half_brick<S>(a, entry, half, lane);
+  for (int half = w & split; half < 2; half += 1 + split) integrate_half_brick<S>(a, entry, half, lane);
 }
 
 // Persistent: every warp takes `chunk` half-bricks of the list(s) per step until they are
@@ -478,15 +478,21 @@ uint32_t plan_blocks(const IntArgs& a) {
 // two (B200, back to back, events included): 64^3 18.5 / 27.2 us, 128^3 21.5 / 26.8, 160^3
 // 26.4 / 29.4, 192^3 33.0 / 31.3, 256^3 53 / 41.  The line lies between 160^3 and 192^3.
 constexpr int kSmallBricks = 8192;
+// Up to this many bricks a warp takes half a brick: the launch is one wave either way and bound by
+// a warp's chain, so testing every brick twice costs less than the second half.  Device us with
+// a warp per brick / per half: 80 x 52 x 80 11.0 / 8.8, 81^3 11.2 / 9.7, 108^3 11.0 / 10.3, 91 x 124
+// x 124 (3,072 bricks) 10.7 / 9.9, 129 x 132 x 205 (7,514) 15.7 / 18.7.
+constexpr int kSplitBricks = 3072;
 
 int brick_count(const IntArgs& a) { return a.bx * a.by * a.bz; }
 
 cudaError_t launch_int_small(int storage, cudaStream_t st, const IntArgs& a) {
-  const int grid = (brick_count(a) + 7) / 8;
+  const int split = brick_count(a) <= kSplitBricks ? 1 : 0;
+  const int grid = ((brick_count(a) << split) + 7) / 8;
   switch (storage) {
-    case KF_STORAGE_F32F32: integrate_small_kernel<KF_STORAGE_F32F32><<<grid, 256, 0, st>>>(a); break;
-    case KF_STORAGE_F16U16: integrate_small_kernel<KF_STORAGE_F16U16><<<grid, 256, 0, st>>>(a); break;
-    default: integrate_small_kernel<KF_STORAGE_RG16I><<<grid, 256, 0, st>>>(a); break;
+    case KF_STORAGE_F32F32: integrate_small_kernel<KF_STORAGE_F32F32><<<grid, 256, 0, st>>>(a, split); break;
+    case KF_STORAGE_F16U16: integrate_small_kernel<KF_STORAGE_F16U16><<<grid, 256, 0, st>>>(a, split); break;
+    default: integrate_small_kernel<KF_STORAGE_RG16I><<<grid, 256, 0, st>>>(a, split); break;
   }
   return cudaGetLastError();
 }

@@ -308,7 +308,8 @@ KF_API int kf_get_stream(kf_session* s, void** cuda_stream);
  * fix their work-group sizes, e.g. integrate.cs local_size 32x32, raycast.cs 32x32) -----
  * Every shape computes bit-identical results; only the time differs. */
 typedef struct kf_launch_shape {
-  int32_t integrate_z_chunk; /* voxels per thread along z: 8, 16 (default) or 32 */
+  int32_t integrate_z_chunk; /* 8, 16 (default) or 32: integrate's warps take 1, 2 or 4    */
+                             /* half-bricks (8 x 8 x 4 voxels) of its plan per step     */
   int32_t raycast_rows;      /* raycast tile of 32 x rows pixels: 2, 4 (default) or 8;  */
                              /* 1 = persistent sweep, every warp taking the next 32-pixel */
                              /* row segment from a queue (sessions only, not batches)     */

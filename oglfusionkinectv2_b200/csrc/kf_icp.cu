@@ -64,7 +64,7 @@ struct IcpArgs {
 };
 
 // A batched launch: the blocks of entry e (one session each) are those whose map word
-// names e; every entry runs its own levels, iterations and grid barrier.
+// names e; every entry runs its own levels, iterations and rows.
 struct IcpBatch {
   const IcpArgs* args;        // per entry
   const uint32_t* block_map;  // per block: entry << 24 | blocks of the entry << 12 | index

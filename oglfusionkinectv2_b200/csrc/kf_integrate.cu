@@ -475,7 +475,7 @@ uint32_t plan_blocks(const IntArgs& a) {
 }
 
 // Volumes of at most this many bricks take the one-launch form.  Per call, one launch against
-// two (B200, back to back, events included): 64^3 18.5 / 27.2 us, 128^3 21.5 / 26.8, 160^3
+// two (B200, a warp per brick, back to back, events included): 64^3 18.5 / 27.2 us, 128^3 21.5 / 26.8, 160^3
 // 26.4 / 29.4, 192^3 33.0 / 31.3, 256^3 53 / 41.  The line lies between 160^3 and 192^3.
 constexpr int kSmallBricks = 8192;
 // Up to this many bricks a warp takes half a brick: the launch is one wave either way and bound by

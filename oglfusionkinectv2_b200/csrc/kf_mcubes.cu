@@ -286,6 +286,9 @@ __global__ void __launch_bounds__(32 * kGenWarps) histo_generate_kernel(McArgs a
   load_counts(s_nt);
   uint16_t* list = s_list[warp];
   for_each_part(a, 4, [&](int tx, int ty, int tz, const uint8_t* tile, int part) {
+    // a tile's bricks past the volume may have no place in the counts: at most 8 voxels a side
+    // make one count, at most 16 eight, and the first codes of the four parts are 0, 1, 8 and 9
+    if (32 * tx + 8 * part >= a.nx) return;
     const uint32_t code = morton_xzy(4 * tx + part, ty, tz), total = __ldg(a.counts + code), off = __ldg(a.offsets + code);
     if (!total || off + total > a.cap || off + total < off) return;  // none, or it does not fit
     const int bx = 32 * tx + 8 * part, by = 8 * ty, bz = 8 * tz;

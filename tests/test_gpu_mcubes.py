@@ -309,3 +309,30 @@ def test_prefix_sums_of_several_threads(threads):
     for t in ts:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("size", [(4, 4, 4), (8, 8, 8), (12, 16, 9), (16, 16, 16), (9, 17, 5), (24, 40, 16)])
+@pytest.mark.parametrize("storage,iso", [(L.KF_STORAGE_F32F32, 0.0), (L.KF_STORAGE_F16U16, 0.25), (L.KF_STORAGE_RG16I, 0.0)])
+def test_soups_of_small_volumes(size, storage, iso):
+    """Volumes narrower than a tile, whose brick counts have fewer than a tile's four bricks of room:
+    a random sign per voxel, so that almost every cube has triangles."""
+    rng = np.random.default_rng(sum(size))
+    n = int(np.prod(size))
+    F = (rng.choice([-1.0, 1.0], n) * rng.uniform(0.3, 1.0, n)).astype(np.float32)
+    W = np.ones(n, np.float32)
+    if storage == L.KF_STORAGE_F32F32:
+        raw = np.concatenate([F, W]).view(np.uint8)
+    elif storage == L.KF_STORAGE_RG16I:
+        raw = np.concatenate([(F * 32766).astype(np.int16), W.astype(np.int16)]).view(np.uint8)
+    else:
+        raw = np.concatenate([F.astype(np.float16).view(np.uint16), W.astype(np.uint16)]).view(np.uint8)
+    cfg = GFusionConfig(volumeSize=size, volumeDimensions=tuple(v / 100.0 for v in size), storage=storage,
+                        quirks=L.KF_QUIRKS_TRACKING & ~(L.KF_Q13_MC_FIRST_SEVEN | L.KF_Q15_MC_BORDER_SKIP))
+    g, o = both(cfg, raw)
+    for method in (L.KF_MC_HISTOPYRAMID, L.KF_MC_SCAN):
+        m, tri = compare(g, o, method, iso)
+        assert tri > n // 4
+        V = m.getVertices()
+        for _ in range(3):  # the same soup from every extraction
+            m.generateMarchingCubes(method)
+            np.testing.assert_array_equal(m.getVertices(), V)

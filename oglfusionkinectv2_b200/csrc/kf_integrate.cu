@@ -284,7 +284,9 @@ __device__ __forceinline__ void integrate_half_brick(const IntArgs& a, uint32_t 
     const float r2 = fmaf(rx, rx, fmaf(ry, ry, 1.0f));
     len[j] = __fmul_rn(r2, mufu_rsqrt(r2));  // sqrt(r2), r2 >= 1
     const bool out = pz[j] < 0.0001f || u < 0.0f || u > fW1 || v < 0.0f || v > fH1;
-    if (j < zend && !out) d[j] = __ldg(a.depth + kf_trunc_index(v, u, (uint32_t)a.W));
+    // a position beyond FP32 makes u or v a NaN, which passes the border test: column or row 0,
+    // as a NaN converts to (fmaxf returns its other operand)
+    if (j < zend && !out) d[j] = __ldg(a.depth + kf_trunc_index(fmaxf(v, 0.0f), fmaxf(u, 0.0f), (uint32_t)a.W));
 #pragma unroll
     for (int r = 0; r < 3; ++r) pos[r] += dz[r];
   }

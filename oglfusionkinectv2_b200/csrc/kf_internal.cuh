@@ -253,7 +253,7 @@ __device__ __forceinline__ uint32_t kf_float_to_u16_trunc(float w) {
   return (uint32_t)__float_as_int(__fadd_rz(w, 8388608.0f)) & 0xFFFFu;  // 0 <= w <= 65535
 }
 
-// (uint32_t)v * w + (uint32_t)u of 0 <= u, v < 2^23, truncated by adds (the conversion
+// (uint32_t)v * w + (uint32_t)u of 0 <= u, v < 2^23 (no NaN), truncated by adds (the conversion
 // instruction runs at a quarter rate); the two offsets leave in one subtraction
 __device__ __forceinline__ uint32_t kf_trunc_index(float v, float u, uint32_t w) {
   const uint32_t bv = (uint32_t)__float_as_int(__fadd_rz(v, 8388608.0f)), bu = (uint32_t)__float_as_int(__fadd_rz(u, 8388608.0f));

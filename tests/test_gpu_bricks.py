@@ -86,3 +86,27 @@ def test_kept_flags_match_rebuilt_flags(storage):
             np.testing.assert_array_equal(a.getVolumeRaw(), b.getVolumeRaw())
             np.testing.assert_array_equal(a.getVerts(), b.getVerts())
             np.testing.assert_array_equal(a.getNorms(), b.getNorms())
+
+
+FAR = np.eye(4)
+FAR[:3, 3] = -1e200, 0.0, -1e200  # finite, but beyond FP32: x / z of every voxel is inf / inf
+
+
+@pytest.mark.parametrize("storage", STORAGES)
+@pytest.mark.parametrize("size", [(33, 20, 17), (64, 64, 64), (170, 165, 161)])
+@pytest.mark.parametrize("pose", [FAR])
+def test_positions_that_are_not_numbers(storage, size, pose):
+    """A voxel whose u is not a number reads column 0 (v is row 212 here), and its distance is not
+    a number either: not above -mu, hence zeroed, unless that pixel holds no depth."""
+    w = small_workload(1, size=64, storage=storage)
+    w.config.volumeSize = size
+    g = GFusion(w.config, w.intrinsics)
+    raw = old_content(size, storage, 7)
+    f = np.full((424, 512), 900.0, np.float32)
+    for d, expect in ((0.0, raw), (900.0, np.zeros_like(raw))):
+        f[212, 0] = d
+        g.setVolumeRaw(raw)
+        g.setPose(pose)
+        g.depthToVertex(f)
+        g.integrate()
+        np.testing.assert_array_equal(g.getVolumeRaw(), expect)

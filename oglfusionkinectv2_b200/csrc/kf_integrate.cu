@@ -108,16 +108,19 @@ __device__ __forceinline__ bool brick_changes(const IntArgs& a, const float* inv
   const float ex = (float)min(KF_BRICK, a.nx - bx * KF_BRICK) * vx, ey = (float)min(KF_BRICK, a.ny - by * KF_BRICK) * vy,
               ez = (float)min(KF_BRICK, a.nz - bz * KF_BRICK) * vz;
   float o[3], ax[3], ay[3], az[3], mag = 0.0f;  // the low corner and the three edges in camera space
+  bool bounded = true;
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     o[r] = inv[r * 4] * wx + inv[r * 4 + 1] * wy + inv[r * 4 + 2] * wz + inv[r * 4 + 3];
     ax[r] = inv[r * 4] * ex;
     ay[r] = inv[r * 4 + 1] * ey;
     az[r] = inv[r * 4 + 2] * ez;
-    mag = fmaxf(mag, fabsf(inv[r * 4]) * a.dimx + fabsf(inv[r * 4 + 1]) * a.dimy + fabsf(inv[r * 4 + 2]) * a.dimz +
-                         fabsf(inv[r * 4 + 3]));
+    const float m = fabsf(inv[r * 4]) * a.dimx + fabsf(inv[r * 4 + 1]) * a.dimy + fabsf(inv[r * 4 + 2]) * a.dimz +
+                    fabsf(inv[r * 4 + 3]);
+    bounded = bounded && m < 1e30f;  // row by row: a maximum would drop a NaN
+    mag = fmaxf(mag, m);
   }
-  if (!(mag < 1e30f)) return true;
+  if (!bounded) return true;
   // outside one of the five half-spaces: the largest value over the corners is negative
   auto top = [&](float kx, float ky, float kz) {
     return kx * o[0] + ky * o[1] + kz * o[2] + fmaxf(0.0f, kx * ax[0] + ky * ax[1] + kz * ax[2]) +

@@ -90,11 +90,13 @@ def test_kept_flags_match_rebuilt_flags(storage):
 
 FAR = np.eye(4)
 FAR[:3, 3] = -1e200, 0.0, -1e200  # finite, but beyond FP32: x / z of every voxel is inf / inf
+MIXED = np.zeros((4, 4))  # not rigid: the inverse's first row is not a number, the others are
+MIXED[:3, 0], MIXED[2, 2], MIXED[:, 3] = (1e200, -1e200, 0.0), 1.0, (1e200, 1e200, -1.0, 1.0)
 
 
 @pytest.mark.parametrize("storage", STORAGES)
 @pytest.mark.parametrize("size", [(33, 20, 17), (64, 64, 64), (170, 165, 161)])
-@pytest.mark.parametrize("pose", [FAR])
+@pytest.mark.parametrize("pose", [FAR, MIXED])
 def test_positions_that_are_not_numbers(storage, size, pose):
     """A voxel whose u is not a number reads column 0 (v is row 212 here), and its distance is not
     a number either: not above -mu, hence zeroed, unless that pixel holds no depth."""

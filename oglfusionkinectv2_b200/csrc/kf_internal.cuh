@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/kf.h"
+#include "kf_solve6.cuh"
 
 #define KF_MAX_LIBRARY 64         // pose library entries kept on the device
 #define KF_TRACK_THREADS 256      // threads per block of the persistent tracking kernels
@@ -450,17 +451,6 @@ __host__ __device__ inline void kf_make_jtj(const double* v21, double* C) {
     }
 }
 
-// 1 / d to FP64 precision without a divide: an FP32 estimate refined by two Newton-Raphson
-// steps y <- y + y (1 - d y), each of which doubles the correct bits (23 -> 46 -> FP64
-// rounding).  Outside FP32's normal range the estimate is the quotient itself.
-__device__ __forceinline__ double kf_rcp_newton(double d) {
-  const double m = fabs(d);
-  double y = (m > 1e-30 && m < 1e30) ? (double)__frcp_rn((float)d) : 1.0 / d;
-  y = fma(fma(-d, y, 1.0), y, y);
-  y = fma(fma(-d, y, 1.0), y, y);
-  return y;
-}
-
 // sin and cos; below |x| = 0.25 by their Taylor series through x^11 and x^12 (the first
 // omitted terms are < 3e-18 relative), which is the whole range of a Gauss-Newton step.
 __device__ __forceinline__ void kf_sincos_step(double x, double* s, double* c) {
@@ -482,52 +472,6 @@ __device__ __forceinline__ void kf_sincos_step(double x, double* s, double* c) {
   } else {
     sincos(x, s, c);
   }
-}
-
-// The inverse of a symmetric 3x3 matrix {m00, m01, m02, m11, m12, m22} by its cofactors.
-__device__ __forceinline__ void kf_inverse3(const double* m, double* r) {
-  const double c00 = fma(m[3], m[5], -m[4] * m[4]), c01 = fma(m[2], m[4], -m[1] * m[5]), c02 = fma(m[1], m[4], -m[2] * m[3]);
-  const double c11 = fma(m[0], m[5], -m[2] * m[2]), c12 = fma(m[1], m[2], -m[0] * m[4]), c22 = fma(m[0], m[3], -m[1] * m[1]);
-  const double i = kf_rcp_newton(fma(m[0], c00, fma(m[1], c01, m[2] * c02)));
-  r[0] = c00 * i; r[1] = c01 * i; r[2] = c02 * i;
-  r[3] = c11 * i; r[4] = c12 * i; r[5] = c22 * i;
-}
-__device__ __forceinline__ double kf_row3(const double* m, int i, double x, double y, double z) {
-  // row i of the symmetric matrix times (x, y, z)
-  return i == 0 ? fma(m[0], x, fma(m[1], y, m[2] * z))
-                : (i == 1 ? fma(m[1], x, fma(m[3], y, m[4] * z)) : fma(m[2], x, fma(m[4], y, m[5] * z)));
-}
-
-// The 6x6 normal equations in FP64 by 3x3 blocks: C = [[A, B], [B^T, D]] (v21: the 21
-// upper-triangular values of reduce.cs rows 7..27), the Schur complement S = D - B^T A^-1 B.
-// For a C that passed the rank check.  The dependent chain is two reciprocals and some thirty
-// multiply-adds; a Cholesky factorisation's six pivots and twelve substitution steps were
-// three times as long (and its error against extended precision slightly larger: 1.7e-16
-// against 1.3e-16 median relative over systems of condition 2 to 3e4).
-__device__ __forceinline__ void kf_solve6(const double* v21, const double* b, double* x) {
-  const double A[6] = {v21[0], v21[1], v21[2], v21[6], v21[7], v21[11]};
-  const double B[3][3] = {{v21[3], v21[4], v21[5]}, {v21[8], v21[9], v21[10]}, {v21[12], v21[13], v21[14]}};
-  const double D[6] = {v21[15], v21[16], v21[17], v21[18], v21[19], v21[20]};
-  double Ai[6], W[3][3], S[6], Si[6], y[3], r[3];
-  kf_inverse3(A, Ai);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) W[i][j] = kf_row3(Ai, i, B[0][j], B[1][j], B[2][j]);  // A^-1 B
-    y[i] = kf_row3(Ai, i, b[0], b[1], b[2]);
-  }
-  int q = 0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-#pragma unroll
-    for (int j = i; j < 3; ++j, ++q) S[q] = fma(-B[0][i], W[0][j], fma(-B[1][i], W[1][j], fma(-B[2][i], W[2][j], D[q])));
-    r[i] = fma(-B[0][i], y[0], fma(-B[1][i], y[1], fma(-B[2][i], y[2], b[3 + i])));
-  }
-  kf_inverse3(S, Si);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) x[3 + i] = kf_row3(Si, i, r[0], r[1], r[2]);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) x[i] = fma(-W[i][0], x[3], fma(-W[i][1], x[4], fma(-W[i][2], x[5], y[i])));
 }
 
 // ---------------------------------------------------------------------------------------

@@ -252,7 +252,9 @@ int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, cudaStream_t 
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return KF_ERR_CUDA;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  // the limit belongs to the kernel in the whole context, so every call sets the same one: a
+  // smaller limit for one tile would refuse the launch that another thread is about to make
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kTile * 4) != cudaSuccess)
     return KF_ERR_CUDA;
   const unsigned grid = (unsigned)std::min<uint64_t>(nt, (uint64_t)kPerSm * sms);
   kernel<<<grid, kThreads, smem, stream>>>(d_in, d_out, n, shift, (uint32_t)nt, w);

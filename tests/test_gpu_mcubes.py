@@ -336,3 +336,36 @@ def test_soups_of_small_volumes(size, storage, iso):
         for _ in range(3):  # the same soup from every extraction
             m.generateMarchingCubes(method)
             np.testing.assert_array_equal(m.getVertices(), V)
+
+
+def test_prefix_sums_of_one_and_many_tiles_at_once():
+    """Half of the threads scan at most one tile, the others many: the two forms of the same kernel's
+    launch must not disturb one another.  Equal alignments, so that all take the same instance."""
+    import threading
+    import torch
+    lib = L.load()
+    wrong = []
+
+    def work(k):
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            n = 16384 - 16 * k if k % 2 else 200_000 + 16 * k
+            x = torch.full((n,), k + 1, dtype=torch.int32, device="cuda")
+            o = torch.empty_like(x)
+            expect = torch.arange(n, dtype=torch.int32, device="cuda") * (k + 1)
+            st.synchronize()
+            for _ in range(300):
+                tot = C.c_uint32()
+                rc = lib.kf_prefix_sum_u32(C.c_void_p(x.data_ptr()), C.c_void_p(o.data_ptr()), n, C.byref(tot),
+                                           C.c_void_p(st.cuda_stream))
+                if rc != L.KF_OK or tot.value != n * (k + 1):
+                    wrong.append((k, rc, tot.value))
+            if not torch.equal(o, expect):
+                wrong.append(k)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not wrong, wrong[:5]

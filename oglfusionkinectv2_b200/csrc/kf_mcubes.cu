@@ -668,9 +668,15 @@ int ensure_soup(kf_session* s, size_t nverts) {
   if (!rc) rc = ensure(s, (void**)&s->d_mc_normals, &s->mc_normal_cap, bytes);
   return rc;
 }
-uint32_t soup_capacity(const kf_session* s) {
-  return (uint32_t)std::min<size_t>(std::min(s->mc_vertex_cap, s->mc_normal_cap) / 16, 0xffffffffu);
+// What the two buffers hold, in units of `vertices` vertices (1, or 3: triangles).  The kernels
+// count units in 32 bits, not bytes or vertices: a soup of more than 2^32 / 3 triangles fits too.
+constexpr uint32_t soup_room(size_t vertex_cap, size_t normal_cap, size_t vertices) {
+  const size_t units = (vertex_cap < normal_cap ? vertex_cap : normal_cap) / (16 * vertices);
+  return units < 0xffffffffu ? (uint32_t)units : 0xffffffffu;
 }
+static_assert(soup_room((size_t)1500000000 * 48, (size_t)1500000000 * 48, 3) == 1500000000u &&
+                  soup_room((size_t)1 << 36, (size_t)1 << 37, 1) == 0xffffffffu && soup_room(95, 960, 3) == 1,
+              "an extraction repeats until its count fits");
 
 // Words of an extraction's tile list: the slots, the list, its length.
 size_t list_words(const McArgs& a) { return 2 * tile_count(a) + 1; }
@@ -733,7 +739,7 @@ int histopyramid(kf_session* s, float iso, uint32_t* n_tri) {
   // and the triangle count (glGetTexImage of the top texel at mcubes.cpp:290-300)
   if ((rc = scan_counts(s, a.counts, offs, codes, offs + codes, sw, s->h_u32_scalar))) return rc;
   for (;;) {
-    a.cap = soup_capacity(s) / 3;
+    a.cap = soup_room(s->mc_vertex_cap, s->mc_normal_cap, 3);
     a.out = s->d_mc_vertices;
     a.nout = s->d_mc_normals;
     if (a.out && a.nout) KF_MC_LAUNCH(histo_generate_kernel, gen_blocks(s), kGenThreads, a);
@@ -770,7 +776,7 @@ int classic(kf_session* s, float iso, uint32_t* n_tri) {
   KF_MC_LAUNCH(classic_classify_kernel, walk_blocks(s), 256, a);
   if ((rc = scan_counts(s, a.counts, offs, n, offs + n, sw, s->h_u32_scalar))) return rc;
   for (;;) {
-    a.cap = soup_capacity(s);
+    a.cap = soup_room(s->mc_vertex_cap, s->mc_normal_cap, 1);
     a.out = s->d_mc_vertices;
     a.nout = s->d_mc_normals;
     if (a.out && a.nout) KF_MC_LAUNCH(classic_generate_kernel, gen_blocks(s), kGenThreads, a);

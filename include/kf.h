@@ -280,10 +280,11 @@ KF_API int kf_intensity_projection(kf_session* s, float* rgba);
 KF_API int kf_save_volume(kf_session* s, const char* path);
 KF_API int kf_load_volume(kf_session* s, const char* path);
 /* Self-test of the bounded device waits: one block waits at a two-block grid barrier that
- * the other block never reaches; after budget_cycles (1e3 .. 1e9 SM clocks) the wait gives
- * up, records the timeout in the session's device error word and the kernel ends.  Returns
- * KF_ERR_TIMEOUT, exactly as a tracking call whose barrier timed out would, and clears the
- * error word; the session stays usable. */
+ * the other block never reaches, then for an ICP reduction row of two blocks of which one
+ * never adds its sums, then for a prefix-sum tile that is never published; after
+ * budget_cycles (1e3 .. 1e9 SM clocks) each wait gives up and its kernel ends.  Returns
+ * KF_ERR_TIMEOUT, exactly as a tracking call whose wait timed out would, and clears the
+ * error word (KF_ERR_STATE when one of the waits did not give up); the session stays usable. */
 KF_API int kf_selftest_barrier_timeout(kf_session* s, long long budget_cycles);
 KF_API int kf_get_pose_library_size(kf_session* s, int* n);
 /* Device times in milliseconds of the last call of each stage, in the order

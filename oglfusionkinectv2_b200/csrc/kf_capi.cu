@@ -1271,12 +1271,25 @@ __global__ void barrier_timeout_selftest_kernel(unsigned* counter, int* error, l
 
 int kf_selftest_barrier_timeout(kf_session* s, long long budget_cycles) {
   if (!s || budget_cycles < 1000 || budget_cycles > KF_BARRIER_SPIN_CYCLES) return KF_ERR_INVALID_ARGUMENT;
-  KF_CUDA_TRY(s, cudaMemsetAsync(s->d_u32_scalar, 0, sizeof(uint32_t), s->stream));
-  barrier_timeout_selftest_kernel<<<2, 32, 0, s->stream>>>(s->d_u32_scalar, &s->d_state->error, budget_cycles);
+  uint32_t* w = s->d_u32_scalar;  // the barrier's counter, whether the row's and the look-back's waits gave up
+  KF_CUDA_TRY(s, cudaMemsetAsync(w, 0, 3 * sizeof(uint32_t), s->stream));
+  barrier_timeout_selftest_kernel<<<2, 32, 0, s->stream>>>(w, &s->d_state->error, budget_cycles);
   KF_CUDA_TRY(s, cudaGetLastError());
   kf_note_launch(s);
+  int rc = kf_launch_icp_wait_selftest(s, reinterpret_cast<int*>(w + 1), budget_cycles);
+  // a look takes some 1,000 cycles; the second reduction row is still zero
+  if (!rc) rc = kf_launch_scan_wait_selftest(kf_icp_words(s->d_state) + KF_ICP_ROW_WORDS, w + 2,
+                                             (uint32_t)(budget_cycles / 1000), s->stream);
+  if (rc) return rc;
+  kf_note_launch(s);
+  KF_CUDA_TRY(s, cudaMemcpyAsync(s->h_u32_scalar, w, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
   // the host side of every tracking call: read the sticky error word, report and clear it
-  return pull_state_head(s);
+  rc = pull_state_head(s);
+  if (rc != KF_ERR_TIMEOUT) return rc;
+  if (s->h_u32_scalar[1] != 1 || s->h_u32_scalar[2] != 1)
+    return fail(s, KF_ERR_STATE, s->h_u32_scalar[1] != 1 ? "the wait for a reduction row did not give up"
+                                                         : "the wait for a tile's sum did not give up");
+  return rc;
 }
 
 int kf_get_cum_twist(kf_session* s, double t[6]) {

@@ -169,10 +169,10 @@ __device__ __forceinline__ void arrive(unsigned long long* row) {
 }
 
 // Sum `lane` of a reduction row once all nb blocks have added theirs; the whole warp waits for
-// all 32 sums.  Bounded: after KF_BARRIER_SPIN_CYCLES, or when another block has given up, the
-// error is recorded and false returned.
-__device__ __forceinline__ bool wait_sum(KfDevState* st, const unsigned long long* row, int lane, unsigned nb,
-                                         unsigned active, long long* sum) {
+// all 32 sums.  Bounded: after `budget` cycles, or when another block has given up, the error is
+// recorded and false returned.
+__device__ __forceinline__ bool wait_sum(int* error, const unsigned long long* row, int lane, unsigned nb, unsigned active,
+                                         long long budget, long long* sum) {
   const unsigned long long mask = (1ull << 48) - 1ull;
   unsigned long long lo = 0, hi = 0;
   const long long t0 = clock64();
@@ -184,13 +184,21 @@ __device__ __forceinline__ bool wait_sum(KfDevState* st, const unsigned long lon
       break;
     __nanosleep(100);
     if ((n & 63u) == 0) {
-      const bool late = clock64() - t0 > KF_BARRIER_SPIN_CYCLES;
-      if (late && lane == 0) atomicExch(&st->error, KF_DEV_ERR_TIMEOUT);
-      if (__any_sync(0xffffffffu, late || *(volatile int*)&st->error)) return false;
+      const bool late = clock64() - t0 > budget;
+      if (late && lane == 0) atomicExch(error, KF_DEV_ERR_TIMEOUT);
+      if (__any_sync(0xffffffffu, late || *(volatile int*)error)) return false;
     }
   }
   *sum = (long long)((((hi & mask) - (hi >> 48) * 0x80000000ull) << 32) + (lo & mask));
   return true;
+}
+
+// Self-test: a row of two blocks of which one never adds its sums.
+__global__ void wait_sum_selftest_kernel(unsigned long long* row, int* error, long long budget) {
+  const int lane = threadIdx.x;
+  add_sum(row, lane, lane);
+  long long sum = 0;
+  wait_sum(error, row, lane, 2u, 2u, budget, &sum);
 }
 
 constexpr int kWarps = KF_TRACK_THREADS / 32;
@@ -480,7 +488,7 @@ __global__ void __launch_bounds__(KF_TRACK_THREADS, 2) icp_kernel(IcpArgs a_one,
       if (warp < 3) {
         if (warp == 0) {
           long long sum = 0;
-          const bool got = wait_sum(st, row, lane, nb, active, &sum);
+          const bool got = wait_sum(&st->error, row, lane, nb, active, KF_BARRIER_SPIN_CYCLES, &sum);
           s_sums[lane] = (double)sum * kInvFix;
           if (lane == 0) s_flag = got ? 1 : 0;
         }
@@ -712,6 +720,14 @@ int kf_launch_icp(kf_session* s, int frame_policy, bool words_zero) {
     KF_CUDA_TRY(s, cudaLaunchKernelEx(&cfg, icp_kernel<1, false>, a, none));
   else
     KF_CUDA_TRY(s, cudaLaunchKernelEx(&cfg, icp_kernel<0, false>, a, none));
+  kf_note_launch(s);
+  return KF_OK;
+}
+
+int kf_launch_icp_wait_selftest(kf_session* s, int* error, long long budget) {
+  KF_CUDA_TRY(s, kf_clear_icp_words(s->d_state, s->stream));
+  wait_sum_selftest_kernel<<<1, 32, 0, s->stream>>>(kf_icp_words(s->d_state), error, budget);
+  KF_CUDA_TRY(s, cudaGetLastError());
   kf_note_launch(s);
   return KF_OK;
 }

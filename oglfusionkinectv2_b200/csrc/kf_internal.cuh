@@ -856,6 +856,11 @@ inline cudaError_t kf_clear_icp_words(KfDevState* st, cudaStream_t stream) {
   return cudaMemsetAsync(kf_icp_words(st), 0, KF_ICP_WORDS * 8, stream);
 }
 
+// Self-tests of the waits for other blocks' words: each leaves the word it is given set to 1 when
+// the wait has given up.
+int kf_launch_icp_wait_selftest(kf_session* s, int* error, long long budget);
+int kf_launch_scan_wait_selftest(const unsigned long long* zero, uint32_t* gave_up, uint32_t max_looks, cudaStream_t stream);
+
 // Count kernels launched outside graph capture (captured graphs are counted per replay).
 inline void kf_note_launch(kf_session* s, int n = 1) {
   if (!s->capturing) s->launches += (uint64_t)n;

@@ -61,8 +61,10 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane) {
   return v;
 }
 
-// Sum of all tiles before `tile`, by one warp.
-__device__ __forceinline__ uint32_t look_back(const unsigned long long* status, uint32_t tile, int lane, uint32_t* gave_up) {
+// Sum of all tiles before `tile`, by one warp.  Bounded: after max_looks looks that found nothing
+// new, or when another wait gave up, *gave_up is set.
+__device__ __forceinline__ uint32_t look_back(const unsigned long long* status, uint32_t tile, int lane, uint32_t* gave_up,
+                                              uint32_t max_looks) {
   uint32_t sum = 0, looks = 0;
   for (int64_t last = (int64_t)tile - 1;;) {  // the nearest tile that is not yet in the sum
     unsigned long long st[kLooks];
@@ -94,7 +96,7 @@ __device__ __forceinline__ uint32_t look_back(const unsigned long long* status, 
     if (!taken) {
       // a wait that gave up (the words were overwritten) ends the others as well
       const bool over = *reinterpret_cast<volatile uint32_t*>(gave_up) != 0;
-      if (++looks > kMaxLooks || __any_sync(0xffffffffu, over)) {
+      if (++looks > max_looks || __any_sync(0xffffffffu, over)) {
         if (lane == 0) atomicExch(gave_up, 1u);
         break;
       }
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, kPerSm)
         if (lane < kWarps) s_pre[k & 1][lane] = inc - w;
       }
       if (prev < ntiles) {
-        const uint32_t base = prev ? look_back(status, prev, lane, scratch + 1) : 0u;
+        const uint32_t base = prev ? look_back(status, prev, lane, scratch + 1, kMaxLooks) : 0u;
         if (lane == 0) {
           if (prev) put_status(status + prev, kPrefix | (uint32_t)(base + sum));
           s_base = base;
@@ -231,6 +233,11 @@ __global__ void __launch_bounds__(kThreads, kPerSm)
   }
 }
 
+// Self-test: the look-back of the second tile, whose first is never published (*status is 0).
+__global__ void look_back_selftest_kernel(const unsigned long long* status, uint32_t* gave_up, uint32_t max_looks) {
+  look_back(status, 1u, threadIdx.x, gave_up, max_looks);
+}
+
 uint64_t tiles(uint64_t n) { return (n + kTile - 1) / kTile; }
 
 }  // namespace
@@ -258,6 +265,11 @@ int kf_scan_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, cudaStream_t 
     return KF_ERR_CUDA;
   const unsigned grid = (unsigned)std::min<uint64_t>(nt, (uint64_t)kPerSm * sms);
   kernel<<<grid, kThreads, smem, stream>>>(d_in, d_out, n, shift, (uint32_t)nt, w);
+  return cudaGetLastError() == cudaSuccess ? KF_OK : KF_ERR_CUDA;
+}
+
+int kf_launch_scan_wait_selftest(const unsigned long long* zero, uint32_t* gave_up, uint32_t max_looks, cudaStream_t stream) {
+  look_back_selftest_kernel<<<1, 32, 0, stream>>>(zero, gave_up, std::min(max_looks, kMaxLooks));
   return cudaGetLastError() == cudaSuccess ? KF_OK : KF_ERR_CUDA;
 }
 

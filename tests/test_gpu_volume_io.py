@@ -166,3 +166,31 @@ def test_copy_into_untouched_memory(voxels):
         assert g.lib.kf_copy_volume_to_host(g._h, C.c_void_p(buf.ctypes.data + off), n) == L.KF_OK
         np.testing.assert_array_equal(buf[off:off + n], raw)
         assert off == 0 or (buf[off - 1] == 77 and buf[off + n] == 78)
+
+
+@pytest.mark.parametrize("jtj", [L.KF_JTJ_FP32, L.KF_JTJ_SPLIT_BF16])
+def test_every_wait_gives_up_and_its_users_go_on(jtj):
+    """The grid barrier, the wait for an ICP row and the prefix sum's look-back each run out (a wait
+    that does not gives another status); ICP frames, the extraction's prefix sum and the scan itself
+    then give what a session that never ran the self-test gives."""
+    import time
+    import torch
+    from oglfusionkinectv2_b200 import MCubes
+    w = small_workload(4, size=64, jtj=jtj)
+    a, b = GFusion(w.config, w.intrinsics), GFusion(w.config, w.intrinsics)
+    for s in (a, b):
+        s.Reset(w.poses[0])
+    for k in range(4):
+        t0 = time.perf_counter()
+        assert a.selftestBarrierTimeout(10 ** (3 + k)) == L.KF_ERR_TIMEOUT
+        assert time.perf_counter() - t0 < 1.0  # 10^6 cycles are half a millisecond
+        assert _run(a, w, [k]) == _run(b, w, [k])
+    np.testing.assert_array_equal(a.getPose(), b.getPose())
+    np.testing.assert_array_equal(a.getVolumeRaw(), b.getVolumeRaw())
+    ma, mb = MCubes(a), MCubes(b)
+    assert ma.generateMarchingCubes() == mb.generateMarchingCubes() > 0
+    np.testing.assert_array_equal(ma.getVertices(), mb.getVertices())
+    x = torch.ones(100_000, dtype=torch.int32, device="cuda")
+    o = torch.empty_like(x)
+    assert a.lib.kf_prefix_sum_u32(x.data_ptr(), o.data_ptr(), x.numel(), None, None) == L.KF_OK
+    assert torch.equal(o, torch.arange(100_000, dtype=torch.int32, device="cuda"))

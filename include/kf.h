@@ -310,7 +310,9 @@ KF_API int kf_get_stream(kf_session* s, void** cuda_stream);
  * Every shape computes bit-identical results; only the time differs. */
 typedef struct kf_launch_shape {
   int32_t integrate_z_chunk; /* 8, 16 (default) or 32: integrate's warps take 1, 2 or 4    */
-                             /* half-bricks (8 x 8 x 4 voxels) of its plan per step     */
+                             /* half-bricks (8 x 8 x 4 voxels) of its plan per step;     */
+                             /* a session of at most 8,192 bricks of 8^3 has no plan and  */
+                             /* no use for it (kf_autotune then keeps 16); batches have    */
   int32_t raycast_rows;      /* raycast tile of 32 x rows pixels: 2, 4 (default) or 8;  */
                              /* 1 = persistent sweep, every warp taking the next 32-pixel */
                              /* row segment from a queue (sessions only, not batches)     */

@@ -1399,6 +1399,8 @@ int kf_autotune(kf_session* s, int repeats, kf_launch_shape* chosen, float* time
   // as in the frame loop, whose volume traffic leaves L2 as a frame's raycast finds it
   // (raycasts back to back would find the previous one's bricks in L2 and favour other
   // shapes).
+  // A volume whose integrate has no chunk is timed once for all three and keeps the default.
+  const bool chunked = kf_integrate_has_chunk(s);
   float best[7] = {1e30f, 1e30f, 1e30f, 1e30f, 1e30f, 1e30f, 1e30f};
   auto elapsed = [&](float* ms) {
     if (cudaEventRecord(e1, s->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
@@ -1409,6 +1411,7 @@ int kf_autotune(kf_session* s, int repeats, kf_launch_shape* chosen, float* time
   for (int round = 0; round < 2 && !rc; ++round)
     for (int c = 0; c < 7 && !rc; ++c) {
       const bool ray = c >= 3;
+      if (!ray && c != 1 && !chunked) continue;
       const int v = ray ? kf_tune_ray_rows[c - 3] : kf_tune_int_zc[c];
       auto launch = [&]() {
         return ray ? kf_launch_raycast_shape(s, v, &t) : kf_launch_integrate_shape(s, 0, v, &t);
@@ -1436,6 +1439,7 @@ int kf_autotune(kf_session* s, int repeats, kf_launch_shape* chosen, float* time
   if (e1) cudaEventDestroy(e1);
   kf_scratch_free(&t);
   if (rc) return rc;
+  if (!chunked) best[0] = best[2] = best[1];
   int zi = 1, ri = 5;  // the defaults (z-chunk 16, 32 x 4 tiles) win ties
   for (int c = 0; c < 3; ++c)
     if (best[c] < best[zi]) zi = c;

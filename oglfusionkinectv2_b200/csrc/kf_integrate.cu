@@ -528,9 +528,12 @@ IntArgs retarget(IntArgs a, const kf_scratch_target* t) {
 
 }  // namespace
 
+// Whether the session's integrate takes the listed form, the only one that has a chunk.
+bool kf_integrate_has_chunk(const kf_session* s) { return s->bx * s->by * s->bz > kSmallBricks; }
+
 int kf_launch_integrate_shape(kf_session* s, int gated, int zc, const kf_scratch_target* t) {
   const IntArgs a = retarget(make_int_args(s, gated), t);
-  if (brick_count(a) <= kSmallBricks) {
+  if (!kf_integrate_has_chunk(s)) {
     KF_CUDA_TRY(s, launch_int_small(s->cfg.storage, s->stream, a));
     kf_note_launch(s);
     return KF_OK;

@@ -882,6 +882,7 @@ int kf_launch_sdf_policy(kf_session* s);
 int kf_launch_integrate(kf_session* s, int gated);
 int kf_launch_raycast(kf_session* s);
 int kf_launch_integrate_shape(kf_session* s, int gated, int zc, const kf_scratch_target* t);
+bool kf_integrate_has_chunk(const kf_session* s);
 int kf_launch_raycast_shape(kf_session* s, int rows, const kf_scratch_target* t);
 inline bool kf_valid_int_zc(int zc) { return zc == 8 || zc == 16 || zc == 32; }
 // raycast shapes: 32 x rows tiles (2, 4, 8), or 1 = the persistent sweep (sessions only)

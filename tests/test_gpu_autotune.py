@@ -116,3 +116,21 @@ def test_batch_autotune_keeps_results_exact():
         for s, t in zip(batched, alone):
             _assert_same(_state(s), _state(t))
 
+
+@pytest.mark.parametrize("size", [(64, 64, 64), (160, 160, 160), (161, 160, 160)])
+def test_integrate_candidates_are_timed_where_they_differ(size):
+    """At most 8,192 bricks: one launch without a chunk, timed once, the default kept.  One brick
+    more along x: three candidates."""
+    w = small_workload(1, size=64, storage=L.KF_STORAGE_F16U16)
+    w.config.volumeSize = size
+    g = GFusion(w.config, w.intrinsics)
+    g.Reset(w.poses[0])
+    g.frameStep(w.frame(0))
+    for _ in range(3):
+        shape, times = g.autotune(repeats=2)
+        z = [times["integrate_z8"], times["integrate_z16"], times["integrate_z32"]]
+        assert all(0 < t < 100 for t in z)
+        if size[0] < 161:
+            assert shape[0] == 16 and len(set(z)) == 1
+        else:
+            assert shape[0] in (8, 16, 32) and len(set(z)) > 1

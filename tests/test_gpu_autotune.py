@@ -134,3 +134,29 @@ def test_integrate_candidates_are_timed_where_they_differ(size):
             assert shape[0] == 16 and len(set(z)) == 1
         else:
             assert shape[0] in (8, 16, 32) and len(set(z)) > 1
+
+
+@pytest.mark.parametrize("storage", [L.KF_STORAGE_F32F32, L.KF_STORAGE_F16U16, L.KF_STORAGE_RG16I])
+def test_every_chunk_of_the_listed_form_is_bit_identical(storage):
+    """9,702 bricks, none of the sides a multiple of one: a session's own plan and list with chunks of
+    8, 16 and 32, and the batch's, over five frames."""
+    w = small_workload(5, size=64, storage=storage, quirks=L.KF_QUIRKS_TRACKING, jtj=L.KF_JTJ_SPLIT_BF16)
+    w.config.volumeSize = (170, 165, 161)
+    frames = [w.frame(k) for k in range(w.n_frames)]
+    ref = None
+    for zc in (8, 16, 32, None):
+        g = GFusion(w.config, w.intrinsics)
+        g.setLaunchShape(zc or 16, 4)
+        g.Reset(w.poses[0])
+        batch = None if zc else GFusionBatch(1)
+        for f in frames:
+            if zc:
+                g.frameStep(f)
+            else:
+                batch.frameStep([g], [f])
+        st = _state(g)
+        if ref is None:
+            ref = st
+            assert (st[2][..., 3] > 0).mean() > 0.2
+        else:
+            _assert_same(st, ref)

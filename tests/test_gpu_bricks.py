@@ -112,3 +112,26 @@ def test_positions_that_are_not_numbers(storage, size, pose):
         g.depthToVertex(f)
         g.integrate()
         np.testing.assert_array_equal(g.getVolumeRaw(), expect)
+
+
+@pytest.mark.parametrize("storage", STORAGES)
+def test_kept_flags_match_rebuilt_flags_in_the_listed_form(storage):
+    """As above for 12,075 bricks, whose integrate takes the plan and its list; 20 frames, across a
+    refresh of the flags."""
+    w = small_workload(20, size=72, storage=storage, quirks=L.KF_QUIRKS_TRACKING)
+    w.config.volumeSize = (200, 163, 180)
+    a, b = GFusion(w.config, w.intrinsics), GFusion(w.config, w.intrinsics)
+    for k in range(20):
+        pose = w.poses[k].copy()
+        pose[:3, 3] += 0.3 * np.sin(0.4 * k) * pose[:3, 2]
+        f = w.frame(k)
+        b.setVolumeRaw(b.getVolumeRaw())
+        for s in (a, b):
+            s.setPose(pose)
+            s.depthToVertex(f)
+            s.integrate()
+            s.raycast()
+        if k % 5 == 4:
+            np.testing.assert_array_equal(a.getVolumeRaw(), b.getVolumeRaw())
+            np.testing.assert_array_equal(a.getVerts(), b.getVerts())
+            np.testing.assert_array_equal(a.getNorms(), b.getNorms())

@@ -56,7 +56,6 @@ __constant__ int c_bourke[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
 __constant__ int c_bourke_edge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6},
                                          {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
 
-constexpr uint32_t kNoSlot = 0xffffffffu;
 constexpr int kTileCubes = 32 * 8 * 8;
 
 // The three extractions: histoPyramid (y/z-swapped corner order), classic, welded mesh.
@@ -70,7 +69,6 @@ struct McArgs {
   const unsigned long long* neg;  // NEG bits; null: every tile is looked at
   int wx, wy;
   int tx, ty, tz;        // tiles of 32 x 8 x 8 cubes
-  uint32_t* slots;       // per tile: its place in the list, kNoSlot for the others
   uint32_t* list;        // the listed tiles
   uint32_t* listed;      // their number
   uint8_t* cases;        // case index per cube, kTileCubes bytes per listed tile (z, y, x)
@@ -122,7 +120,6 @@ __global__ void __launch_bounds__(256) tile_list_kernel(McArgs a) {
   if (lane == 0 && m) at = atomicAdd(a.listed, (uint32_t)__popc(m));
   at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
   if (on) a.list[at] = t;
-  if (t < n) a.slots[t] = on ? at : kNoSlot;
 }
 
 // A warp's share of the listed tiles' work, `parts` parts each, in turn over the grid.
@@ -678,8 +675,8 @@ static_assert(soup_room((size_t)1500000000 * 48, (size_t)1500000000 * 48, 3) == 
                   soup_room((size_t)1 << 36, (size_t)1 << 37, 1) == 0xffffffffu && soup_room(95, 960, 3) == 1,
               "an extraction repeats until its count fits");
 
-// Words of an extraction's tile list: the slots, the list, its length.
-size_t list_words(const McArgs& a) { return 2 * tile_count(a) + 1; }
+// Words of an extraction's tile list: the list, its length.
+size_t list_words(const McArgs& a) { return tile_count(a) + 1; }
 
 // The list that belongs to the case bytes of histopyramid() and classic().
 uint32_t* case_tiles(const kf_session* s, const McArgs& a) {
@@ -689,9 +686,8 @@ uint32_t* case_tiles(const kf_session* s, const McArgs& a) {
 // Lays the list out at w, zeroes its length and fills it.
 int list_tiles(kf_session* s, McArgs* a, uint32_t* w) {
   const size_t n = tile_count(*a);
-  a->slots = w;
-  a->list = w + n;
-  a->listed = w + 2 * n;
+  a->list = w;
+  a->listed = w + n;
   KF_CUDA_TRY(s, cudaMemsetAsync(a->listed, 0, 4, s->stream));
   tile_list_kernel<<<(int)((n + 255) / 256), 256, 0, s->stream>>>(*a);
   KF_CUDA_TRY(s, cudaGetLastError());
@@ -926,7 +922,7 @@ int kf_mc_copy_base_level(kf_session* s, uint32_t* base, uint64_t count) {
   } catch (const std::bad_alloc&) {
     return KF_ERR_OUT_OF_MEMORY;
   }
-  KF_CUDA_TRY(s, cudaMemcpyAsync(list.data(), case_tiles(s, a) + tiles, (tiles + 1) * 4, cudaMemcpyDeviceToHost, s->stream));
+  KF_CUDA_TRY(s, cudaMemcpyAsync(list.data(), case_tiles(s, a), (tiles + 1) * 4, cudaMemcpyDeviceToHost, s->stream));
   KF_CUDA_TRY(s, cudaStreamSynchronize(s->stream));
   const size_t listed = list[tiles];
   try {

@@ -491,7 +491,7 @@ KF_API int kf_prefix_sum_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, 
  * budget or inside a host framework that owns every device allocation, where the
  * scratch that kf_prefix_sum_u32 allocates for more than 2^28 elements, or when many threads
  * call it at once, is not allowed.  Same result as
- * kf_prefix_sum_u32; the scratch is a 262,220-byte array compiled into the library,
+ * kf_prefix_sum_u32; the scratch is a 131,136-byte array compiled into the library,
  * which every GPU that loads the library keeps until the process exits.
  *   - n may be at most 2^28 (268,435,456) elements; larger n returns KF_ERR_CAPACITY.
  *   - The first call in a CUDA context looks up the array's device address (a host-side

@@ -276,19 +276,18 @@ int kf_launch_scan_wait_selftest(const unsigned long long* zero, uint32_t* gave_
 // ---- scratch without allocations --------------------------------------------------------
 // An allocation per call costs 0.4-0.9 ms: the driver's pool gives its memory back at every
 // synchronisation.  So both entry points keep their scratch in arrays compiled into the library,
-// sized for KF_NOALLOC_SCAN_MAX_ELEMENTS elements (2^28 make 16,385 tiles: 32,776 words):
-//  - kf_prefix_sum_u32_noalloc has one array (65,555 words, 262,220 bytes), shared by all its
-//    calls on a device;
+// of KF_SCAN_WORDS words, which KF_NOALLOC_SCAN_MAX_ELEMENTS elements need (2^28 make 16,385
+// tiles: 32,776 words):
+//  - kf_prefix_sum_u32_noalloc has one array (131,136 bytes), shared by all its calls on a device;
 //  - kf_prefix_sum_u32 waits for its result, so a call borrows one of a few slots and returns
 //    it at the end; when none is free, the input is larger or the stream is being captured, the
 //    scratch is allocated.
-// Every GPU that loads this library holds the arrays (0.8 MB) until the process exits.
+// Every GPU that loads this library holds the arrays (0.66 MB) until the process exits.
 #define KF_NOALLOC_SCAN_MAX_ELEMENTS (1ull << 28)
-#define KF_NOALLOC_SCAN_WORDS 65555
+#define KF_SCAN_WORDS 32784
 #define KF_SCAN_SLOTS 4
-#define KF_SCAN_SLOT_WORDS 32784
-static __device__ __align__(256) uint32_t g_noalloc_scan_scratch[KF_NOALLOC_SCAN_WORDS];
-static __device__ __align__(256) uint32_t g_scan_slots[KF_SCAN_SLOTS * KF_SCAN_SLOT_WORDS];
+static __device__ __align__(256) uint32_t g_noalloc_scan_scratch[KF_SCAN_WORDS];
+static __device__ __align__(256) uint32_t g_scan_slots[KF_SCAN_SLOTS * KF_SCAN_WORDS];
 
 namespace {
 std::mutex g_scratch_mu;
@@ -382,7 +381,7 @@ uint32_t* borrow_slot(unsigned long long* ctx_id, int* slot) {
       e->busy |= 1u << k;
       *ctx_id = e->ctx_id;
       *slot = k;
-      return e->slots + (size_t)k * KF_SCAN_SLOT_WORDS;
+      return e->slots + (size_t)k * KF_SCAN_WORDS;
     }
   return nullptr;
 }
@@ -403,7 +402,7 @@ extern "C" int kf_prefix_sum_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t
   unsigned long long ctx_id = 0;
   int slot = -1;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (words <= KF_SCAN_SLOT_WORDS && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+  if (words <= KF_SCAN_WORDS && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
       capture == cudaStreamCaptureStatusNone)
     scratch = borrow_slot(&ctx_id, &slot);
   if (!scratch && cudaMallocAsync((void**)&scratch, words * sizeof(uint32_t), st) != cudaSuccess) {
@@ -438,7 +437,7 @@ extern "C" int kf_prefix_sum_u32_noalloc(const uint32_t* d_in, uint32_t* d_out, 
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)cuda_stream;
   const uint32_t* result = nullptr;
-  rc = kf_scan_u32(d_in, d_out, n, st, scratch, KF_NOALLOC_SCAN_WORDS, &result);
+  rc = kf_scan_u32(d_in, d_out, n, st, scratch, KF_SCAN_WORDS, &result);
   if (rc || !total) return rc;
   uint32_t h[2] = {0, 0};
   if (cudaMemcpyAsync(h, result, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -502,7 +502,10 @@ KF_API int kf_prefix_sum_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n, 
  *     (different streams, or host threads) race and corrupt each other's results.
  *     Serialise them, e.g. on one stream.
  *   - No cudaMalloc/cudaFree or allocating library call is made; if total is not NULL the
- *     call copies it back and synchronises the stream. */
+ *     call copies it back and synchronises the stream.
+ *   - A tile waits for the sums before it, some 0.2 s at most.  A call whose wait gave up (the
+ *     scratch was overwritten by an overlapping call) returns KF_ERR_CUDA; with total NULL
+ *     nothing is read back, and the caller cannot learn of it. */
 KF_API int kf_prefix_sum_u32_noalloc(const uint32_t* d_in, uint32_t* d_out, uint64_t n,
                                      uint32_t* total, void* cuda_stream);
 

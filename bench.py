@@ -213,6 +213,9 @@ def algorithmic_bytes(cfg, stage):
 
 
 def stage_rooflines(w, per, peak):
+    """Per stage: `achieved` and `frac` are the dense byte model over the stage's time, which is not
+    traffic (the kernels visit only what a frame can change, so it can exceed the peak);
+    `traffic_gbs` and `traffic_frac` are the DRAM bytes of an ncu capture, where there is one."""
     out = {}
     for stage in ("integrate", "raycast", "track"):
         ms = per.get(stage) or 0.0
@@ -221,9 +224,10 @@ def stage_rooflines(w, per, peak):
         algo = algorithmic_bytes(w.config, stage)
         gbs = algo / (ms / 1000.0) / 1e9
         traffic = measured_traffic(w.name, stage)
-        out[stage] = {"algorithmic_bytes": algo, "ms": ms, "achieved": gbs, "frac": gbs / peak,
-                      "traffic": traffic,
-                      "traffic_frac": (traffic / (ms / 1000.0) / 1e9 / peak if traffic else None)}
+        traffic_gbs = traffic / (ms / 1000.0) / 1e9 if traffic else None
+        out[stage] = {"algorithmic_bytes": algo, "ms": ms, "achieved": gbs, "frac": gbs / peak, "of": "dense byte model",
+                      "traffic": traffic, "traffic_gbs": traffic_gbs,
+                      "traffic_frac": (traffic_gbs / peak if traffic else None)}
     return out
 
 
@@ -863,11 +867,12 @@ def main():
                        "launch_shape": tuned or {"integrate_z_chunk": (fixed or (16, 4))[0],
                                                  "raycast_rows": (fixed or (16, 4))[1], "autotune": "off"}},
             "stage_ms": per, "stage_frames": stage_frames,
-            # achieved: the DRAM bytes the kernel really moves (ncu capture) over its time; the dense
-            # byte model (every voxel read and written once) is a bound that no frame comes near,
-            # since only the bricks it can change are visited, and stands beside it
-            "roofline": {"kernel": dom, "bound": "hbm", "achieved": traffic_gbs or dense_gbs, "peak": peak,
-                         "unit": "GB/s", "frac": ((traffic_gbs or dense_gbs) / peak if dense_gbs else None),
+            # achieved: the DRAM bytes the kernel really moves (ncu capture) over its time, null for a
+            # workload without a capture.  The dense byte model (every voxel read and written once)
+            # stands beside it without a fraction: only the bricks that a frame can change are
+            # visited, so it is not traffic and can exceed the peak
+            "roofline": {"kernel": dom, "bound": "hbm", "achieved": traffic_gbs, "peak": peak,
+                         "unit": "GB/s", "frac": (traffic_gbs / peak if traffic_gbs else None),
                          "peak_source": peak_kind, "algorithmic_bytes": algo, "dense_model_gbs": dense_gbs,
                          "traffic": traffic,
                          "traffic_gbs": traffic_gbs,

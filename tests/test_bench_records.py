@@ -61,3 +61,14 @@ def test_plain_workloads_and_metric(bench):
 def test_launch_shape_flag(bench):
     a = args(bench, "--launch-shape", "32,4")
     assert tuple(int(x) for x in a.launch_shape.split(",")) == (32, 4)
+
+
+def test_stage_traffic_is_apart_from_the_byte_model(bench):
+    """Fractions of the peak come from captured DRAM bytes alone; a stage without a capture has none."""
+    per = {"integrate": 0.05, "raycast": 0.06, "track": 0.08}
+    captured = bench.stage_rooflines(bench.workload(args(bench), 4), per, 6000.0)["integrate"]
+    assert captured["of"] == "dense byte model"
+    assert captured["traffic_gbs"] == pytest.approx(captured["traffic"] / 0.05e-3 / 1e9)
+    assert captured["traffic_frac"] == pytest.approx(captured["traffic_gbs"] / 6000.0) and captured["traffic_frac"] < 1
+    none = bench.stage_rooflines(bench.workload(args(bench, "--workload", "c1"), 4), per, 6000.0)["integrate"]
+    assert none["traffic_gbs"] is None and none["traffic_frac"] is None
